@@ -215,8 +215,10 @@ TWMC_API int64_t twmc_launch_count(const twmc_handle* h);
  * square stencil / Lieb neighbour table), "rowrun_kernel" (square stencil,
  * 4096 sites, FP32 Philox runs), "lieb_cell_kernel" (Lieb lattice, even
  * number of cells), "ell_cluster_pow2_kernel" / "ell_cluster_kernel" (square
- * stencil above 8192 sites on 2-CTA clusters). Kernels chosen at launch time
- * are reported after the first step. */
+ * stencil above 8192 sites). FP32 Philox runs of the square stencil go by the
+ * name of their size class, whichever kernel (packed pairs of sites, or the
+ * unpacked one) runs them. Kernels chosen at launch time are reported after
+ * the first step. */
 TWMC_API const char* twmc_kernel_name(const twmc_handle* h);
 /* The CUDA stream (cudaStream_t) all of the handle's work is issued on, for
  * callers that order their own work or record events against it. */
@@ -250,10 +252,10 @@ typedef struct twmc_hbatch twmc_hbatch;
  * takes one step variant -- "fft" (register FFT: chains of 32..1024 sites,
  * 16x16, 32x32, 64x64), "ell2" / "ell4" / "ell8" (real-space stencil with 2,
  * 4, 8 sites per thread, 256-thread CTAs, up to 512 / 1024 / 2048 sites),
- * "rowrun" (runs of four sites along a row, 512-thread CTAs, ny a multiple
- * of 4, up to 4096 sites), "ell8w" (8 sites per thread, 512-thread CTAs, up
- * to 4096 sites), "cluster_pow2" / "cluster" (2-CTA clusters, 4097..16384
- * sites; the power-of-two form for N = 2^k, ny a power of two <= N/4) --
+ * "rowrun" (8 sites per thread, 512-thread CTAs, ny a multiple of 4, up to
+ * 4096 sites), "ell8w" (8 sites per thread, 512-thread CTAs, up to 4096
+ * sites), "cluster_pow2" / "cluster" (CTA clusters, 4097..16384 sites; the
+ * first for N = 2^k, ny a power of two <= N/4) --
  * and every (point, trajectory group) is a work item of a persistent
  * work-queue kernel for its CTA geometry, taken from an atomic counter,
  * longest items first. One frame (frame_steps steps of every point, FP64

@@ -463,6 +463,7 @@ int advance(twmc_handle* h, int64_t n, bool want_nk, int64_t t0 = 0, int64_t t1 
   a.nbr_w = h->d_nbr_w.p;
   a.J = h->J;
   a.f_J = float(h->J);
+  fill_pair_constants(&a);
   a.lieb_pbc = h->pbc;
   a.lieb_jab = h->J_AB;
   a.lieb_jbc = h->J_BC;

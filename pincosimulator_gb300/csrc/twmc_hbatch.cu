@@ -4,14 +4,14 @@
 // Each point is a square lattice (1-D chain or 2-D) with uniform parameters
 // and its own trajectories, and takes one step variant: the register FFT
 // (plans of 32..1024-site chains and 16x16, 32x32, 64x64), the real-space
-// stencil with 2, 4 or 8 sites per thread, row runs of four sites, or the
-// 2-CTA cluster stencil above 4096 sites. Every (point, trajectory group) is
-// a work item of a persistent work-queue kernel -- one per CTA geometry:
-// hbatch_kernel (256 threads), hbatch_kernel_512 and hbatch_cluster_kernel
-// (2-CTA clusters of 1024 threads) -- whose CTAs take items from an atomic
+// stencil with 2, 4 or 8 sites per thread, or a cluster of CTAs above 4096
+// sites. Every (point, trajectory group) is a work item of a persistent
+// work-queue kernel -- one per CTA geometry: hbatch_kernel (256 threads),
+// hbatch_kernel_512, hbatch_cluster4_kernel (clusters of four 256-thread CTAs)
+// and hbatch_cluster_kernel (of two 1024-thread CTAs) -- whose CTAs take items from an atomic
 // counter, longest item first, and run the variant's step body for that
 // point (arguments and tables reloaded into shared memory when the point
-// changes). One frame -- counter reset, the three queues on parallel graph
+// changes). One frame -- counter reset, the queues on parallel graph
 // branches, the batched FP64 moments and the advance of every point's
 // Philox step counter -- is captured once into a CUDA graph and replayed per
 // frame; the per-point arguments live in device memory so the replayed graph
@@ -19,7 +19,7 @@
 //
 // Autotuner: for every shape, the first batch that needs it times each
 // variant the shape admits (FFT plan, real-space stencil with 2 / 4 / 8
-// sites per thread -- i.e. trajectories per CTA --, row runs, cluster forms)
+// sites per thread -- i.e. trajectories per CTA --, cluster forms)
 // on a trial batch of that point alone and keeps the fastest; choices are
 // cached per device and shape in a JSON file ($TWMC_TUNE_CACHE, default
 // ~/.cache/twmc_tune.json).
@@ -40,6 +40,7 @@
 
 #include "twmc.h"
 #include "twmc_moments.cuh"
+#include "twmc_pair.cuh"
 #include "twmc_square.cuh"
 
 namespace twmc {
@@ -98,19 +99,40 @@ __device__ __forceinline__ void hb_run(unsigned char* smem, const StepArgs& a, b
   g.run(a, group, buf);
 }
 
-// Step variants of a batch point. Each runs in one of three persistent
+// Step variants of a batch point. Each runs in one of four persistent
 // work-queue kernels, by CTA geometry: 256 threads (register-FFT plans and
-// real-space stencils with 2, 4 or 8 sites per thread), 512 threads (row
-// runs, 8 sites per thread) and 2-CTA clusters of 1024 threads (lattices
-// above 4096 sites).
+// real-space stencils with 2, 4 or 8 sites per thread), 512 threads (8 sites
+// per thread, "rowrun" and "ell8w") and, for lattices above 4096 sites,
+// clusters: 4 CTAs of 256 threads where the packed form splits that way, else
+// 2 CTAs of 1024 threads. Real-space points run the packed body
+// (twmc_pair.cuh) wherever their lattice pairs up and splits into their
+// variant's threads, else the unpacked bodies.
 enum HbVariant : int {
   kVarFft = 0, kVarEll2, kVarEll4, kVarEll8, kVarRowrun, kVarEll8w, kVarClusterPow2, kVarCluster, kVarCount
 };
 constexpr const char* kVarName[kVarCount] = {"fft", "ell2", "ell4", "ell8", "rowrun", "ell8w", "cluster_pow2",
                                              "cluster"};
-enum HbQueue : int { kQ256 = 0, kQ512, kQCluster, kQueues };
+enum HbQueue : int { kQ256 = 0, kQ512, kQCluster, kQCluster4, kQueues };
 constexpr int kVarQueue[kVarCount] = {kQ256, kQ256, kQ256, kQ256, kQ512, kQ512, kQCluster, kQCluster};
-constexpr int kQueueCta[kQueues] = {256, 512, 1024};
+constexpr int kQueueCta[kQueues] = {256, 512, 1024, 256};
+
+// The packed body's split of a real-space point: V rows per block, NB blocks
+// per thread, chain or not, CTAs per trajectory; 0 = the unpacked body.
+struct PairSplit {
+  int v = 0, nb = 0, cl = 1;
+  bool chain = false;
+  int64_t rows = 0, ny = 0;  // of one CTA
+  int code() const { return v == 0 ? 0 : (chain ? 4096 : 0) + cl * 256 + v * 16 + nb; }
+  int tpt() const { return int((rows / v * ny + nb - 1) / nb); }
+};
+#define TWMC_HB_CODE(V, NB, CH, CL) ((CH ? 4096 : 0) + CL * 256 + V * 16 + NB)
+// Splits of the 256- and 512-thread queues, preferred first for their slots
+// per thread (V NB): longer runs of rows load less.
+#define TWMC_HB_SPLITS_256(X)                                                            \
+  X(1, 1, false) X(2, 1, false) X(1, 2, false) X(4, 1, false) X(2, 2, false) X(1, 4, false) \
+  X(1, 1, true) X(2, 1, true) X(1, 2, true) X(4, 1, true) X(1, 4, true)
+#define TWMC_HB_SPLITS_512(X) X(2, 2, false) X(4, 1, false) X(1, 4, false) X(4, 1, true) X(1, 4, true)
+
 constexpr int64_t kOneGroup = int64_t(1) << 62;  // group stride past any batch: a body runs exactly one group
 
 // Fetches the next work item (point, trajectory group) of a queue into
@@ -156,17 +178,26 @@ hbatch_kernel(const StepArgs* __restrict__ pts, const int* __restrict__ pvar, co
           default: break;
         }
         break;
-      case kVarEll2: ell_body<float, 2, HB_CTA, 1, true>(s_a, smem_raw, w.y, kOneGroup); break;
-      case kVarEll4: ell_body<float, 4, HB_CTA, 1, true>(s_a, smem_raw, w.y, kOneGroup); break;
-      case kVarEll8: ell_body<float, 8, HB_CTA, 1, true>(s_a, smem_raw, w.y, kOneGroup); break;
-      default: break;
+      default:
+        switch (pshape[w.x]) {
+#define TWMC_HB_CASE(V, NB, CH) \
+  case TWMC_HB_CODE(V, NB, CH, 1): pair_body<V, NB, CH, PAIR_SCALAR>(s_a, smem_raw, w.y); break;
+          TWMC_HB_SPLITS_256(TWMC_HB_CASE)
+#undef TWMC_HB_CASE
+          default:
+            switch (pvar[w.x]) {
+              case kVarEll2: ell_body<float, 2, HB_CTA, 1, true>(s_a, smem_raw, w.y, kOneGroup); break;
+              case kVarEll4: ell_body<float, 4, HB_CTA, 1, true>(s_a, smem_raw, w.y, kOneGroup); break;
+              default: ell_body<float, 8, HB_CTA, 1, true>(s_a, smem_raw, w.y, kOneGroup); break;
+            }
+        }
     }
   }
 }
 
-// 512-thread queue: row runs of four sites and the 8-site real-space stencil.
+// 512-thread queue: eight sites per thread.
 __global__ void __launch_bounds__(512, 1)
-hbatch_kernel_512(const StepArgs* __restrict__ pts, const int* __restrict__ pvar, const int2* __restrict__ items,
+hbatch_kernel_512(const StepArgs* __restrict__ pts, const int* __restrict__ pshape, const int2* __restrict__ items,
                   int nitems, int* __restrict__ counter) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(16) StepArgs s_a;
@@ -175,26 +206,29 @@ hbatch_kernel_512(const StepArgs* __restrict__ pts, const int* __restrict__ pvar
   int2 w;
   bool reload;
   while (hb_next(pts, items, nitems, counter, s_a, s_item, cur, w, reload)) {
-    if (pvar[w.x] == kVarRowrun) rowrun_body<512>(s_a, smem_raw, w.y, kOneGroup);
-    else ell_body<float, 8, 512, 1, true>(s_a, smem_raw, w.y, kOneGroup);
+    switch (pshape[w.x]) {
+#define TWMC_HB_CASE(V, NB, CH) \
+  case TWMC_HB_CODE(V, NB, CH, 1): pair_body<V, NB, CH, PAIR_SCALAR>(s_a, smem_raw, w.y); break;
+      TWMC_HB_SPLITS_512(TWMC_HB_CASE)
+#undef TWMC_HB_CASE
+      default: ell_body<float, 8, 512, 1, true>(s_a, smem_raw, w.y, kOneGroup); break;
+    }
   }
 }
 
-// Cluster queue: one item is one trajectory, run by both CTAs of a 2-CTA
-// cluster; rank 0 takes the item and rank 1 reads it through distributed
-// shared memory, so both ranks leave the loop together.
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(1024, 1)
-hbatch_cluster_kernel(const StepArgs* __restrict__ pts, const int* __restrict__ pvar,
-                      const int2* __restrict__ items, int nitems, int* __restrict__ counter) {
+// Cluster queues: one item is one trajectory, run by all CTAs of a cluster;
+// rank 0 takes the item and the others read it through distributed shared
+// memory, so that all ranks leave the loop together.
+template <int CL, class Run>
+__device__ __forceinline__ void hb_cluster_loop(const StepArgs* __restrict__ pts, const int2* __restrict__ items,
+                                                int nitems, int* __restrict__ counter, StepArgs& s_a, int& s_item,
+                                                Run run) {
   namespace cg = cooperative_groups;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ __align__(16) StepArgs s_a;
-  __shared__ int s_item;
   cg::cluster_group cl = cg::this_cluster();
   const unsigned rank = cl.block_rank();
   int cur = -1;
   for (;;) {
-    cl.sync();  // both ranks are done with the previous item (buffers, peer reads, s_item)
+    cl.sync();  // every rank is done with the previous item (buffers, peer accesses, s_item)
     if (rank == 0 && threadIdx.x == 0) s_item = atomicAdd(counter, 1);
     cl.sync();
     const int it = rank == 0 ? s_item : *cl.map_shared_rank(&s_item, 0);
@@ -202,15 +236,46 @@ hbatch_cluster_kernel(const StepArgs* __restrict__ pts, const int* __restrict__ 
     const int2 w = items[it];
     if (w.x != cur) {
       __syncthreads();
-      for (int i = threadIdx.x; i < int(sizeof(StepArgs) / 4); i += 1024)
+      for (int i = threadIdx.x; i < int(sizeof(StepArgs) / 4); i += blockDim.x)
         reinterpret_cast<uint32_t*>(&s_a)[i] = reinterpret_cast<const uint32_t*>(pts + w.x)[i];
       __syncthreads();
       cur = w.x;
     }
-    if (pvar[w.x] == kVarClusterPow2) ell_cluster_pow2_body<1024, true>(s_a, smem_raw, w.y, kOneGroup);
-    else ell_cluster_body<float, 1024>(s_a, smem_raw, w.y, kOneGroup);
+    run(w);
   }
-  cl.sync();  // rank 0's shared memory stays until rank 1 has read the last item index
+  cl.sync();  // rank 0's shared memory stays until the others have read the last item index
+}
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(1024, 1)
+hbatch_cluster_kernel(const StepArgs* __restrict__ pts, const int* __restrict__ pvar, const int* __restrict__ pshape,
+                      const int2* __restrict__ items, int nitems, int* __restrict__ counter) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ __align__(16) StepArgs s_a;
+  __shared__ int s_item;
+  hb_cluster_loop<2>(pts, items, nitems, counter, s_a, s_item, [&](int2 w) {
+    switch (pshape[w.x]) {
+      case TWMC_HB_CODE(4, 1, false, 2): pair_body<4, 1, false, PAIR_SCALAR, 2>(s_a, smem_raw, w.y); break;
+      case TWMC_HB_CODE(5, 1, false, 2): pair_body<5, 1, false, PAIR_SCALAR, 2>(s_a, smem_raw, w.y); break;
+      case TWMC_HB_CODE(3, 1, false, 2): pair_body<3, 1, false, PAIR_SCALAR, 2>(s_a, smem_raw, w.y); break;
+      case TWMC_HB_CODE(1, 1, false, 2): pair_body<1, 1, false, PAIR_SCALAR, 2>(s_a, smem_raw, w.y); break;
+      default:
+        if (pvar[w.x] == kVarClusterPow2) ell_cluster_pow2_body<1024, true>(s_a, smem_raw, w.y, kOneGroup);
+        else ell_cluster_body<float, 1024>(s_a, smem_raw, w.y, kOneGroup);
+    }
+  });
+}
+
+// Clusters of four 256-thread CTAs, two CTAs per SM: while one waits at its
+// cluster barrier the other computes (128x128 4.15e11 site-updates/s against
+// 3.24e11 on two 1024-thread CTAs).
+__global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(256, 2)
+hbatch_cluster4_kernel(const StepArgs* __restrict__ pts, const int2* __restrict__ items, int nitems,
+                       int* __restrict__ counter) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ __align__(16) StepArgs s_a;
+  __shared__ int s_item;
+  hb_cluster_loop<4>(pts, items, nitems, counter, s_a, s_item,
+                     [&](int2 w) { pair_body<8, 1, false, PAIR_SCALAR, 4>(s_a, smem_raw, w.y); });
 }
 
 // FP64 moment blocks of every point: grid (site chunk, block, point).
@@ -337,15 +402,16 @@ struct twmc_hbatch {
   cudaStream_t s0 = nullptr;
   // the 512-thread and cluster queues run on their own captured streams,
   // parallel graph branches beside the 256-thread queue on s0
-  cudaStream_t sq[kQueues] = {nullptr, nullptr, nullptr};
+  cudaStream_t sq[kQueues] = {};
   cudaEvent_t fork = nullptr, e0 = nullptr, e1 = nullptr;
-  cudaEvent_t qjoin[kQueues] = {nullptr, nullptr, nullptr};
+  cudaEvent_t qjoin[kQueues] = {};
   std::string err;
   int64_t frame_steps = 1;
   size_t npts = 0;
   std::vector<twmc_point_desc> desc;
   std::vector<int> var;            // step variant (HbVariant) per point
-  std::vector<int> shape;          // register-FFT plan id per point (kVarFft), else -1
+  std::vector<int> shape;          // register-FFT plan id per point (kVarFft), else its PairSplit code
+  std::vector<PairSplit> split;    // of the real-space points
   std::vector<std::string> plan;
   std::vector<int64_t> nsites, ntraj, off_state, nblocks;
   DBuf<float2> state;
@@ -357,8 +423,8 @@ struct twmc_hbatch {
   DBuf<StepArgs> args;
   DBuf<int> pvar, pshape;
   DBuf<int2> qitems[kQueues];
-  int qn[kQueues] = {0, 0, 0}, qgrid[kQueues] = {0, 0, 0};
-  size_t qsmem[kQueues] = {0, 0, 0};
+  int qn[kQueues] = {}, qgrid[kQueues] = {};
+  size_t qsmem[kQueues] = {};
   DBuf<int> counter;               // one work counter per queue
   DBuf<MomentArgs> margs;
   DBuf<double> moments;
@@ -440,11 +506,12 @@ void fill_args(const twmc_hbatch* b, size_t i, StepArgs* a) {
   a->f_kn = float(-2.0 * M_LN2 * d.gamma * d.dt / 4.0);
   a->noise_mode = TWMC_NOISE_PHILOX;
   a->nsites = d.nx * d.ny;
-  a->nx = d.nx;
-  a->ny = d.ny;
+  a->nx = d.ny == 1 ? 1 : d.nx;  // a chain is one row whichever side it lies on
+  a->ny = d.ny == 1 ? d.nx : d.ny;
   a->hop_kind = 1;
   a->J = d.J;
   a->f_J = float(d.J);
+  fill_pair_constants(a);
 }
 
 
@@ -467,32 +534,75 @@ bool var_ok(int v, const twmc_point_desc& d) {
   }
 }
 
+// The packed split of a real-space point in variant v, or none: lattices that
+// pair up by whole rows (or chains of an even length) whose blocks fit the
+// variant's threads and shared memory.
+PairSplit var_split(int v, const twmc_point_desc& d) {
+  PairSplit best;
+  const int64_t n = d.nx * d.ny;
+  const bool chain = d.nx == 1 || d.ny == 1;
+  if (v == kVarFft || n < 2 || n % 2 || (!chain && d.nx % 2)) return best;
+  const int64_t ny = chain ? 1 : d.ny, rows = n / 2 / ny;
+  constexpr size_t kMostSmem = 200 * 1024;
+  auto consider = [&](int rv, int nb, bool ch, int cl, int cta) {
+    if (best.v || ch != chain || rows % (int64_t(rv) * cl)) return;
+    PairSplit s;
+    s.v = rv; s.nb = nb; s.cl = cl; s.chain = ch; s.rows = rows / cl; s.ny = ny;
+    const int64_t tpt = s.tpt();
+    if (tpt > cta) return;
+    const size_t per = 2 * pair_buffer_bytes(ch, rv, s.rows, ny) * size_t(cl > 1 ? 1 : cta / tpt);
+    if (per <= kMostSmem) best = s;
+  };
+  const int slots = v == kVarEll2 ? 1 : v == kVarEll4 ? 2 : 4;
+  switch (kVarQueue[v]) {
+    case kQ256:
+      for (int want : {slots, 4})
+#define TWMC_HB_TRY(V, NB, CH) if (V * NB == want) consider(V, NB, CH, 1, 256);
+      { TWMC_HB_SPLITS_256(TWMC_HB_TRY) }
+#undef TWMC_HB_TRY
+      break;
+    case kQ512:
+#define TWMC_HB_TRY(V, NB, CH) consider(V, NB, CH, 1, 512);
+      TWMC_HB_SPLITS_512(TWMC_HB_TRY)
+#undef TWMC_HB_TRY
+      break;
+    default:
+      consider(8, 1, false, 4, 256);
+      for (int rv : {4, 5, 3, 1}) consider(rv, 1, false, 2, 1024);
+  }
+  return best;
+}
+
+// Queue of a point.
+int var_queue(int v, const PairSplit& s) { return s.v && s.cl == 4 ? kQCluster4 : kVarQueue[v]; }
+
 // Threads per trajectory of the real-space variants, and trajectories per
 // work item of every variant.
-int var_tpt(int v, int64_t n) {
+int var_tpt(int v, int64_t n, const PairSplit& s) {
+  if (s.v) return s.tpt();
   const int64_t half = (n + 1) / 2;
   switch (v) {
     case kVarEll2: return int(half);
     case kVarEll4: return int((half + 1) / 2);
-    case kVarEll8: case kVarEll8w: return int((half + 3) / 4);
-    case kVarRowrun: return int(n / 8);
+    case kVarEll8: case kVarEll8w: case kVarRowrun: return int((half + 3) / 4);
     default: return 0;
   }
 }
-int var_tpc(int v, const twmc_point_desc& d, int shape) {
+int var_tpc(int v, const twmc_point_desc& d, int shape, const PairSplit& s) {
   if (v == kVarFft) return hb_tpc(shape);
   if (v == kVarClusterPow2 || v == kVarCluster) return 1;
-  return kQueueCta[kVarQueue[v]] / var_tpt(v, d.nx * d.ny);
+  return kQueueCta[kVarQueue[v]] / var_tpt(v, d.nx * d.ny, s);
 }
 // Dynamic shared memory of one item of variant v.
-size_t var_smem(int v, const twmc_point_desc& d, int shape) {
+size_t var_smem(int v, const twmc_point_desc& d, int shape, const PairSplit& s) {
   const int64_t n = d.nx * d.ny;
   if (v == kVarFft) return kHbSmem;
+  if (s.v) return 2 * pair_buffer_bytes(s.chain, s.v, s.rows, s.ny) * size_t(var_tpc(v, d, shape, s));
   if (v == kVarClusterPow2 || v == kVarCluster) {
     const int64_t half = (n + 1) / 2, q = (half + 1) / 2;
     return sizeof(float2) * 4 * size_t(q);
   }
-  return ell_state_bytes(true, var_tpc(v, d, shape), n, sizeof(float2));
+  return ell_state_bytes(true, var_tpc(v, d, shape, s), n, sizeof(float2));
 }
 
 // The variant a point takes without tuning: the register FFT where a plan
@@ -510,7 +620,7 @@ int default_var(const twmc_point_desc& d) {
     if (!var_ok(v, d)) continue;
     const int vpt = v == kVarEll2 ? 2 : v == kVarEll4 ? 4 : 8;
     const int cta = kQueueCta[kVarQueue[v]];
-    const int64_t tpc = cta / var_tpt(v, n);
+    const int64_t tpc = cta / var_tpt(v, n, PairSplit());
     const double u = double(n * tpc) / double(int64_t(cta) * vpt);
     if (u > best_u + 1e-9) { best_u = u; best = v; }
   }
@@ -568,7 +678,8 @@ int hb_build(twmc_hbatch* b, const twmc_point_desc* points, size_t n, int64_t fr
 
   // step variant per point: forced, tuned (per shape, cached) or the default
   b->var.assign(n, -1);
-  b->shape.assign(n, -1);
+  b->shape.assign(n, 0);
+  b->split.assign(n, PairSplit());
   b->plan.assign(n, "");
   std::map<std::string, std::string> cache;
   const std::string cpath = tune_cache_path();
@@ -600,8 +711,9 @@ int hb_build(twmc_hbatch* b, const twmc_point_desc* points, size_t n, int64_t fr
     if (v < 0 || v >= kVarCount || !var_ok(v, d))
       return hfail(b, TWMC_ERR_INVALID, "point " + std::to_string(i) + ": no step variant for this lattice");
     b->var[i] = v;
-    if (v == kVarFft) b->shape[i] = hb_shape_id(lg2(d.nx), lg2(d.ny));
-    static const char* qname[kQueues] = {"hbatch_kernel", "hbatch_kernel_512", "hbatch_cluster_kernel"};
+    b->split[i] = var_split(v, d);
+    b->shape[i] = v == kVarFft ? hb_shape_id(lg2(d.nx), lg2(d.ny)) : b->split[i].code();
+    static const char* qname[kQueues] = {"hbatch_kernel", "hbatch_kernel_512", "hbatch_cluster_kernel", "hbatch_cluster_kernel"};
     b->plan[i] = std::string(qname[kVarQueue[v]]) + "<" + kVarName[v] + " " + std::to_string(d.nx) + "x" +
                  std::to_string(d.ny) + ">";
   }
@@ -701,12 +813,12 @@ int hb_build(twmc_hbatch* b, const twmc_point_desc* points, size_t n, int64_t fr
     a.nk = v == kVarFft ? b->nk.p + b->off_state[i] : nullptr;  // k-space populations from the FFT only
     a.tw = b->tw.p + tw_off[i];
     a.ktab = b->kt.p + tw_off[i];
-    a.tpt = var_tpt(v, b->nsites[i]);
+    a.tpt = var_tpt(v, b->nsites[i], b->split[i]);
     a.dbuf = 1;
-    const int q = kVarQueue[v];
-    const int tpc = var_tpc(v, points[i], b->shape[i]);
+    const int q = var_queue(v, b->split[i]);
+    const int tpc = var_tpc(v, points[i], b->shape[i], b->split[i]);
     order[q].push_back({double(b->nsites[i]) * double(tpc), i});
-    b->qsmem[q] = std::max(b->qsmem[q], var_smem(v, points[i], b->shape[i]));
+    b->qsmem[q] = std::max(b->qsmem[q], var_smem(v, points[i], b->shape[i], b->split[i]));
     MomentArgs& m = hm[i];
     m.ntraj = b->ntraj[i];
     m.nsites = b->nsites[i];
@@ -722,7 +834,7 @@ int hb_build(twmc_hbatch* b, const twmc_point_desc* points, size_t n, int64_t fr
     std::vector<int2> items;
     for (const auto& o : order[q]) {
       const size_t i = o.second;
-      const int tpc = var_tpc(b->var[i], points[i], b->shape[i]);
+      const int tpc = var_tpc(b->var[i], points[i], b->shape[i], b->split[i]);
       for (int64_t g = 0; g < (b->ntraj[i] + tpc - 1) / tpc; ++g) items.push_back(make_int2(int(i), int(g)));
     }
     b->qn[q] = int(items.size());
@@ -743,7 +855,8 @@ int hb_build(twmc_hbatch* b, const twmc_point_desc* points, size_t n, int64_t fr
   cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, b->device);
   const void* qfn[kQueues] = {reinterpret_cast<const void*>(hbatch_kernel),
                               reinterpret_cast<const void*>(hbatch_kernel_512),
-                              reinterpret_cast<const void*>(hbatch_cluster_kernel)};
+                              reinterpret_cast<const void*>(hbatch_cluster_kernel),
+                              reinterpret_cast<const void*>(hbatch_cluster4_kernel)};
   for (int q = 0; q < kQueues; ++q) {
     if (b->qn[q] == 0) continue;
     const size_t smem = b->qsmem[q];
@@ -751,15 +864,16 @@ int hb_build(twmc_hbatch* b, const twmc_point_desc* points, size_t n, int64_t fr
     cudaError_t e = cudaFuncSetAttribute(qfn[q], cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     if (e != cudaSuccess) { cudaGetLastError(); return hfail(b, TWMC_ERR_CUDA, std::string("batch queue smem: ") + cudaGetErrorString(e)); }
     int slots = 0;
-    if (q == kQCluster) {
+    if (q == kQCluster || q == kQCluster4) {
+      const int cl = q == kQCluster ? 2 : 4;
       cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3(2, 1, 1);
-      cfg.blockDim = dim3(1024, 1, 1);
+      cfg.gridDim = dim3(cl, 1, 1);
+      cfg.blockDim = dim3(kQueueCta[q], 1, 1);
       cfg.dynamicSmemBytes = smem;
       int ncl = 0;
       e = cudaOccupancyMaxActiveClusters(&ncl, qfn[q], &cfg);
       if (e != cudaSuccess || ncl <= 0) { cudaGetLastError(); return hfail(b, TWMC_ERR_CUDA, "batch cluster queue does not fit"); }
-      b->qgrid[q] = 2 * std::min(b->qn[q], ncl);
+      b->qgrid[q] = cl * std::min(b->qn[q], ncl);
     } else {
       e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&slots, qfn[q], kQueueCta[q], smem);
       if (e != cudaSuccess || slots <= 0) { cudaGetLastError(); return hfail(b, TWMC_ERR_CUDA, "batch queue does not fit on an SM"); }
@@ -767,7 +881,7 @@ int hb_build(twmc_hbatch* b, const twmc_point_desc* points, size_t n, int64_t fr
     }
   }
 
-  // capture one frame: counters reset, the three queues on parallel
+  // capture one frame: counters reset, the queues on parallel
   // branches, then the batched moments and the step-counter bump
   cudaStream_t s0 = b->s0;
   cudaStreamSynchronize(s0);
@@ -781,10 +895,13 @@ int hb_build(twmc_hbatch* b, const twmc_point_desc* points, size_t n, int64_t fr
         b->args.p, b->pvar.p, b->pshape.p, b->qitems[kQ256].p, b->qn[kQ256], b->counter.p + kQ256);
   if (b->qn[kQ512] > 0)
     hbatch_kernel_512<<<b->qgrid[kQ512], 512, b->qsmem[kQ512], b->sq[kQ512]>>>(
-        b->args.p, b->pvar.p, b->qitems[kQ512].p, b->qn[kQ512], b->counter.p + kQ512);
+        b->args.p, b->pshape.p, b->qitems[kQ512].p, b->qn[kQ512], b->counter.p + kQ512);
   if (b->qn[kQCluster] > 0)
     hbatch_cluster_kernel<<<b->qgrid[kQCluster], 1024, b->qsmem[kQCluster], b->sq[kQCluster]>>>(
-        b->args.p, b->pvar.p, b->qitems[kQCluster].p, b->qn[kQCluster], b->counter.p + kQCluster);
+        b->args.p, b->pvar.p, b->pshape.p, b->qitems[kQCluster].p, b->qn[kQCluster], b->counter.p + kQCluster);
+  if (b->qn[kQCluster4] > 0)
+    hbatch_cluster4_kernel<<<b->qgrid[kQCluster4], 256, b->qsmem[kQCluster4], b->sq[kQCluster4]>>>(
+        b->args.p, b->qitems[kQCluster4].p, b->qn[kQCluster4], b->counter.p + kQCluster4);
   cudaError_t le = cudaGetLastError();
   for (int q = 0; q < kQueues; ++q) {
     cudaEventRecord(b->qjoin[q], b->sq[q]);
