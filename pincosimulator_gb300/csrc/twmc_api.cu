@@ -101,10 +101,12 @@ struct twmc_handle {
   DevBuf d_work, d_area;
   DevBuf d_wide;           // FP32 -> FP64 download staging (bounded chunk)
   // final-field pipeline of twmc_run: the last steps run in kFinalChunks
-  // trajectory ranges; each range is widened into d_snap and copied to the
-  // host on dl_stream while the next range computes
+  // trajectory ranges, each on a stream of its own; each range is widened into
+  // d_snap and copied to the host on dl_stream while the later ranges compute
   cudaStream_t dl_stream = nullptr;
+  std::vector<cudaStream_t> range_stream;
   std::vector<cudaEvent_t> dl_ev;
+  cudaEvent_t fork = nullptr;
   cudaEvent_t snap_ready = nullptr, snap_free = nullptr;  // d_snap written (stream) / read (dl_stream)
   DevBuf d_snap;
   // page-locked host staging for fields copied row by row to the caller
@@ -407,9 +409,12 @@ std::pair<cudaEvent_t, cudaEvent_t> get_events(twmc_handle* h) {
 
 // Advances the batch by n steps (n may be 0 to refresh the k-space buffer).
 // n steps of trajectories [t0, t1) of the batch (all when t1 < 0); the
-// step counter advances only when `bump` (a caller stepping the batch in
-// several ranges bumps it once).
-int advance(twmc_handle* h, int64_t n, bool want_nk, int64_t t0 = 0, int64_t t1 = -1, bool bump = true) {
+// step counter advances, and the launch is timed, only when `range_stream` is
+// null (a caller stepping the batch in ranges on streams of their own does
+// both once).
+int advance(twmc_handle* h, int64_t n, bool want_nk, int64_t t0 = 0, int64_t t1 = -1,
+            cudaStream_t range_stream = nullptr) {
+  const cudaStream_t stream = range_stream ? range_stream : h->stream;
   if (t1 < 0) t1 = h->ntraj;
   if (t1 <= t0) return TWMC_OK;
   const size_t c2 = 2 * rsize(h->prec), r1 = rsize(h->prec);
@@ -421,6 +426,7 @@ int advance(twmc_handle* h, int64_t n, bool want_nk, int64_t t0 = 0, int64_t t1 
   std::memset(&a, 0, sizeof(a));
   a.state = at(h->d_state.p, row_c);
   a.ntraj = t1 - t0;
+  a.batch_traj = h->ntraj;
   a.nsteps = n;
   a.step0 = h->step_pos;
   a.seeds = h->d_seeds.as<uint32_t>() + t0;
@@ -484,25 +490,30 @@ int advance(twmc_handle* h, int64_t n, bool want_nk, int64_t t0 = 0, int64_t t1 
     return fail(h, TWMC_ERR_INVALID, "noise buffer shorter than the run");
   int nparams = 0;
   for (int k = 0; k < 3; ++k) nparams += (*par[k] != nullptr);
-  auto ev = get_events(h);
-  cudaEventRecord(ev.first, h->stream);
+  std::pair<cudaEvent_t, cudaEvent_t> ev{nullptr, nullptr};
+  if (!range_stream) {
+    ev = get_events(h);
+    cudaEventRecord(ev.first, stream);
+  }
   std::string err;
   bool ok;
   if (h->use_fft) {
-    ok = h->prec == 0 ? square_launch_f32(h->bx, h->by, a, nparams, h->stream, &h->last_info, &err)
-                      : square_launch_f64(h->bx, h->by, a, nparams, h->stream, &h->last_info, &err);
+    ok = h->prec == 0 ? square_launch_f32(h->bx, h->by, a, nparams, stream, &h->last_info, &err)
+                      : square_launch_f64(h->bx, h->by, a, nparams, stream, &h->last_info, &err);
     if (ok) h->kname = h->last_info.name;  // "square_fft_kernel<fast>" for the compiled-in common run
   } else {
-    ok = ell_launch(h->prec, a, h->stream, &h->last_info, &err);
+    ok = ell_launch(h->prec, a, stream, &h->last_info, &err);
     if (ok && (std::strncmp(h->last_info.name, "ell_cluster", 11) == 0 || std::strcmp(h->last_info.name, "lieb_cell_kernel") == 0 ||
                std::strcmp(h->last_info.name, "rowrun_kernel") == 0))
       h->kname = h->last_info.name;
   }
-  cudaEventRecord(ev.second, h->stream);
-  h->ev_pending.push_back(ev);
+  if (!range_stream) {
+    cudaEventRecord(ev.second, stream);
+    h->ev_pending.push_back(ev);
+  }
   if (!ok) return fail(h, TWMC_ERR_CUDA, err);
   ++h->launches;
-  if (bump) h->step_pos += uint32_t(n);
+  if (!range_stream) h->step_pos += uint32_t(n);
   return TWMC_OK;
 }
 
@@ -858,10 +869,13 @@ void twmc_destroy(twmc_handle* h) {
   cudaSetDevice(h->device);
   if (h->stream) cudaStreamSynchronize(h->stream);
   if (h->dl_stream) cudaStreamSynchronize(h->dl_stream);
+  for (cudaStream_t s : h->range_stream) cudaStreamSynchronize(s);
   for (cudaEvent_t e : h->dl_ev) cudaEventDestroy(e);
+  if (h->fork) cudaEventDestroy(h->fork);
   if (h->h_stage) cudaFreeHost(h->h_stage);
   if (h->snap_ready) cudaEventDestroy(h->snap_ready);
   if (h->snap_free) cudaEventDestroy(h->snap_free);
+  for (cudaStream_t s : h->range_stream) cudaStreamDestroy(s);
   if (h->dl_stream) cudaStreamDestroy(h->dl_stream);
   for (auto& e : h->ev_pending) { cudaEventDestroy(e.first); cudaEventDestroy(e.second); }
   for (auto& e : h->ev_free) { cudaEventDestroy(e.first); cudaEventDestroy(e.second); }
@@ -1032,6 +1046,7 @@ int twmc_run(twmc_handle* h, const twmc_task_desc* tasks, size_t n, twmc_outputs
       struct Drain {
         twmc_handle* h;
         ~Drain() {
+          for (cudaStream_t s : h->range_stream) cudaStreamSynchronize(s);
           if (h->stream) cudaStreamSynchronize(h->stream);
           if (h->dl_stream) cudaStreamSynchronize(h->dl_stream);
         }
@@ -1052,8 +1067,13 @@ int twmc_run(twmc_handle* h, const twmc_task_desc* tasks, size_t n, twmc_outputs
       };
       // final-field pipeline: the steps that end the run go in kFinalChunks
       // trajectory ranges, each range widened into d_snap and copied to the
-      // caller's rows on dl_stream while the next range computes (also Philox
-      // noise and no work / area)
+      // caller's rows on dl_stream while the later ranges compute (also Philox
+      // noise and no work / area). The ranges run on streams of their own, so
+      // that one range's CTAs start in the room the previous one leaves as it
+      // drains (one after the other on one stream, each left its last wave
+      // partly empty: 50x50 with 777 trajectories took 2.0 times one launch);
+      // falling priorities keep their order, a range's widening before the
+      // next range's CTAs.
       const bool pipe = stage && out && out->final_field && !h->thermo && h->noise_mode == TWMC_NOISE_PHILOX &&
                         int64_t(bn) >= kFinalChunks;
       bool final_sent = false, frame_sent = false;
@@ -1063,17 +1083,34 @@ int twmc_run(twmc_handle* h, const twmc_task_desc* tasks, size_t n, twmc_outputs
         if (!(pipe && last && nsteps > 0)) return advance(h, nsteps, nk);
         int r2 = stage_setup();
         if (r2) return r2;
+        if (!h->fork) TWMC_CUDA(h, cudaEventCreateWithFlags(&h->fork, cudaEventDisableTiming));
+        int least = 0, greatest = 0;
+        TWMC_CUDA(h, cudaDeviceGetStreamPriorityRange(&least, &greatest));
+        while (h->range_stream.size() < size_t(kFinalChunks)) {
+          cudaStream_t s2;
+          TWMC_CUDA(h, cudaStreamCreateWithPriority(&s2, cudaStreamNonBlocking,
+                                                    std::min(greatest + int(h->range_stream.size()), least)));
+          h->range_stream.push_back(s2);
+        }
         double* snap = h->d_snap.as<double>();
         const float* st = static_cast<const float*>(h->d_state.p);
+        auto ev = get_events(h);
+        h->ev_pending.push_back(ev);
+        TWMC_CUDA(h, cudaEventRecord(ev.first, h->stream));
+        TWMC_CUDA(h, cudaEventRecord(ev.second, h->stream));  // (recorded again below: both stand on every exit)
+        TWMC_CUDA(h, cudaEventRecord(h->fork, h->stream));
         for (int c = 0; c < kFinalChunks; ++c) {
           const int64_t t0 = int64_t(bn) * c / kFinalChunks, t1 = int64_t(bn) * (c + 1) / kFinalChunks;
-          r2 = advance(h, nsteps, nk, t0, t1, false);
+          const cudaStream_t s2 = h->range_stream[size_t(c)];
+          TWMC_CUDA(h, cudaStreamWaitEvent(s2, h->fork, 0));
+          r2 = advance(h, nsteps, nk, t0, t1, s2);
           if (r2) return r2;
-          if (c == 0) TWMC_CUDA(h, cudaStreamWaitEvent(h->stream, h->snap_free, 0));
+          TWMC_CUDA(h, cudaStreamWaitEvent(s2, h->snap_free, 0));
           std::string err;
-          if (!widen_launch(st + size_t(t0) * row, snap + size_t(t0) * row, int64_t(size_t(t1 - t0) * row), h->stream, &err))
+          if (!widen_launch(st + size_t(t0) * row, snap + size_t(t0) * row, int64_t(size_t(t1 - t0) * row), s2, &err))
             return fail(h, TWMC_ERR_CUDA, err);
-          TWMC_CUDA(h, cudaEventRecord(h->dl_ev[size_t(c)], h->stream));
+          TWMC_CUDA(h, cudaEventRecord(h->dl_ev[size_t(c)], s2));
+          TWMC_CUDA(h, cudaStreamWaitEvent(h->stream, h->dl_ev[size_t(c)], 0));
           TWMC_CUDA(h, cudaStreamWaitEvent(h->dl_stream, h->dl_ev[size_t(c)], 0));
           TWMC_CUDA(h, cudaMemcpyAsync(out->final_field + (idx[0] + size_t(t0)) * row, snap + size_t(t0) * row,
                                        size_t(t1 - t0) * row * sizeof(double), cudaMemcpyDeviceToHost, h->dl_stream));
@@ -1082,6 +1119,7 @@ int twmc_run(twmc_handle* h, const twmc_task_desc* tasks, size_t n, twmc_outputs
                                        snap + size_t(t0) * row, row, size_t(t1 - t0), h->dl_stream));
         }
         frame_sent = fdst != nullptr;
+        TWMC_CUDA(h, cudaEventRecord(ev.second, h->stream));
         TWMC_CUDA(h, cudaEventRecord(h->snap_free, h->dl_stream));
         h->step_pos += uint32_t(nsteps);
         final_sent = true;

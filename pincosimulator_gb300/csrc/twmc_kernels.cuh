@@ -38,6 +38,7 @@ struct PairConst {
 struct StepArgs {
   void* state;            // [ntraj][N] complex (R)
   int64_t ntraj;
+  int64_t batch_traj;     // trajectories in flight with this launch's (its batch), for choices of geometry
   int64_t nsteps;         // steps in this launch
   uint32_t step0;         // global index of the first step (Philox counter word 1)
   const uint32_t* seeds;  // [ntraj] Philox key word 0

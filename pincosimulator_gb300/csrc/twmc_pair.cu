@@ -71,7 +71,7 @@ bool pair_plan(const StepArgs& a, PairPlan* best) {
       p.tpc = cl > 1 ? 1 : int(p.threads / tpt);  // as the kernel counts them
       p.smem = buf * size_t(p.tpc);
       if (p.threads > most || int64_t(p.smem) > kSmemPerSm) continue;
-      const double t = step_cycles(p, a.ntraj, sms);
+      const double t = step_cycles(p, std::max(a.ntraj, a.batch_traj), sms);
       if (best_t < 0 || t < best_t) { best_t = t; *best = p; }
     }
   };
