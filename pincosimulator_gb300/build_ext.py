@@ -24,7 +24,7 @@ FLAGS = ["-O3", "-lineinfo", "-std=c++17", "--expt-relaxed-constexpr", "-Xcompil
 SOURCES = ["twmc_api.cu", "twmc_square_f32.cu", "twmc_square_f64.cu", "twmc_ell.cu", "twmc_misc.cu",
            "twmc_noalloc.cu", "twmc_hbatch.cu",
            "twmc_mlp.cu", "twmc_ell_fast.cu", "twmc_pair.cu", "twmc_pair_scalar.cu", "twmc_pair_rsl.cu",
-           "twmc_pair_site.cu"]
+           "twmc_pair_site.cu", "twmc_lieb_pair.cu"]
 
 
 def _write_plans() -> None:

@@ -94,10 +94,11 @@ struct twmc_handle {
   bool timedep = false;
   bool thermo = false;     // work / area accumulators (TWMCThermoSolver)
   int integrator = TWMC_INTEGRATOR_EULER;
-  // every trajectory's per-site rsl has the real part par_scalar[0][0]
-  // (square lattice: Im omega uniform over the base, the disorder and any
-  // given realisations); set by the batch initialisation
-  bool rsl_re_uniform = false;
+  // every trajectory's per-site rsl (iU) has the real part par_scalar[0][0]
+  // (par_scalar[1][0]): Im omega, on the Lieb lattice Im E (Im U) uniform over
+  // the base, the disorder and any given realisations; set by the batch
+  // initialisation
+  bool rsl_re_uniform = false, iU_re_uniform = false;
   DevBuf d_work, d_area;
   DevBuf d_wide;           // FP32 -> FP64 download staging (bounded chunk)
   // final-field pipeline of twmc_run: the last steps run in kFinalChunks
@@ -461,6 +462,7 @@ int advance(twmc_handle* h, int64_t n, bool want_nk, int64_t t0 = 0, int64_t t1 
   a.ktab = h->d_ktab.p;
   a.kfac = h->integrator == TWMC_INTEGRATOR_SPLIT ? h->d_kfac.p : nullptr;
   a.rsl_re_uniform = h->rsl_re_uniform ? 1 : 0;
+  a.iU_re_uniform = h->iU_re_uniform ? 1 : 0;
   a.nsites = h->nsites;
   a.nx = h->lattice == TWMC_LATTICE_SQUARE ? h->nx : 1;
   a.ny = h->lattice == TWMC_LATTICE_SQUARE ? h->ny : h->nsites;
@@ -469,10 +471,10 @@ int advance(twmc_handle* h, int64_t n, bool want_nk, int64_t t0 = 0, int64_t t1 
   a.nbr_w = h->d_nbr_w.p;
   a.J = h->J;
   a.f_J = float(h->J);
-  fill_pair_constants(&a);
   a.lieb_pbc = h->pbc;
   a.lieb_jab = h->J_AB;
   a.lieb_jbc = h->J_BC;
+  fill_pair_constants(&a);
   a.f_lieb_jab = float(h->J_AB);
   a.f_lieb_jbc = float(h->J_BC);
   if (h->timedep) {
@@ -586,24 +588,25 @@ int batch_init(twmc_handle* h, const twmc_task_desc* tasks, size_t n) {
     if (!upload_raw(&h->d_given, g.data(), g.size())) return fail(h, TWMC_ERR_NOMEM, "initial field upload");
     ia.given = h->d_given.as<double>();
   }
-  // Real part of rsl = Im(omega) - gamma/2 the same at every site of every
-  // trajectory: Im of the base uniform, no imaginary disorder amplitude, and
-  // given realisations with that imaginary part (square lattice).
-  {
-    bool uni = h->lattice == TWMC_LATTICE_SQUARE;
-    const Matrix& mo = h->m_omega;
+  // Real part of rsl = Im(omega) - gamma/2 (Lieb: -Im(E) - gamma/2), and of
+  // iU = -Im(U), the same at every site of every trajectory: Im of the base
+  // uniform, no imaginary disorder amplitude, and given realisations with that
+  // imaginary part.
+  auto im_uniform = [&](const Matrix& mo, const double* twmc_task_desc::*given) {
     const double im0 = mo.base.empty() ? 0.0 : mo.base[0].imag();
-    for (const cd& v : mo.base) uni = uni && v.imag() == im0;
+    for (const cd& v : mo.base) if (v.imag() != im0) return false;
     if (mo.kind != TWMC_DISORDER_NONE)
-      for (const cd& v : mo.amp) uni = uni && v.imag() == 0.0;
-    if (tasks[0].omega_realization)
-      for (size_t i = 0; i < n && uni; ++i) {
-        const double* w = tasks[i].omega_realization;
-        if (!w) { uni = false; break; }  // rejected below: all tasks or none
-        for (int64_t j = 0; j < N && uni; ++j) uni = w[2 * j + 1] == im0;
+      for (const cd& v : mo.amp) if (v.imag() != 0.0) return false;
+    if (tasks[0].*given)
+      for (size_t i = 0; i < n; ++i) {
+        const double* w = tasks[i].*given;
+        if (!w) return false;  // rejected below: all tasks or none
+        for (int64_t j = 0; j < N; ++j) if (w[2 * j + 1] != im0) return false;
       }
-    h->rsl_re_uniform = uni;
-  }
+    return true;
+  };
+  h->rsl_re_uniform = im_uniform(h->m_omega, &twmc_task_desc::omega_realization);
+  h->iU_re_uniform = im_uniform(h->m_U, &twmc_task_desc::U_realization);
   // matrices: 0 = U, 1 = omega/E, 2 = F ; per-site parameter buffers: rsl <- omega, iU <- U, iF <- F
   const Matrix* mats[3] = {&h->m_U, &h->m_omega, &h->m_F};
   const uint32_t streams[3] = {kStreamU, kStreamOmega, kStreamF};

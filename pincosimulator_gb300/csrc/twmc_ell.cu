@@ -140,6 +140,8 @@ bool ell_launch(int prec, const StepArgs& a, cudaStream_t s, LaunchInfo* info, s
     if (info) info->name = path_name(a);
     return pair_launch(a, plan, s, info, err);
   }
+  // (F(t) allowed)
+  if (prec == 0 && a.noise_mode == 0 && a.work == nullptr && lieb_pair_ok(a)) return lieb_pair_launch(a, s, info, err);
   if (use_cluster(prec, a)) return cluster_launch(a, s, info, err);
   if (lieb_cell_ok(a)) return prec == 0 ? lieb_cell_launch<float>(a, s, info, err) : lieb_cell_launch<double>(a, s, info, err);
   if (use_fast(prec, a)) return ell_launch_fast_f32(a, s, info, err);

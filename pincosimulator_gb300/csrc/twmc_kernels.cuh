@@ -28,7 +28,8 @@ namespace twmc {
 // Scalar coefficients of the packed real-space step (twmc_pair.cuh), each
 // value in both lanes so that a packed instruction takes it as it is.
 struct PairConst {
-  float2 jt;              // dt J
+  float2 jt;              // dt J (Lieb: dt J_BC)
+  float2 jab;             // Lieb: dt J_AB
   float2 ax, ay, bx, by;  // dt (rsl - iU), dt iU
   float2 fx, fy;          // dt iF
   float2 kn;              // f_kn
@@ -69,6 +70,7 @@ struct StepArgs {
   int kfac_smem;          // split step: 1 = table copied to shared memory, 0 = read from global (L2)
   int rsl_re_uniform;     // per-site rsl with the same real part (-gamma/2 + Im omega) everywhere, equal
                           // to rsl_s[0]: the fast FFT kernel then reads the imaginary parts only
+  int iU_re_uniform;      // the same for a per-site iU and iU_s[0]
   // ell kernel
   int tpt;                // threads per trajectory
   int64_t nsites;         // N
@@ -99,7 +101,8 @@ struct StepArgs {
 // Fills pk from the FP64 scalars (host).
 inline void fill_pair_constants(StepArgs* a) {
   auto both = [](double v) { return make_float2(float(v), float(v)); };
-  a->pk.jt = both(a->dt * a->J);
+  a->pk.jt = both(a->dt * (a->hop_kind == 0 ? a->lieb_jbc : a->J));
+  a->pk.jab = both(a->dt * a->lieb_jab);
   a->pk.ax = both(a->dt * (a->rsl_s[0] - a->iU_s[0]));
   a->pk.ay = both(a->dt * (a->rsl_s[1] - a->iU_s[1]));
   a->pk.bx = both(a->dt * a->iU_s[0]);

@@ -83,14 +83,17 @@ __device__ __forceinline__ PairNoise pair_noise(u32x4 w, float2 kn) {
 // A = dt (rsl - iU), B = dt iU, F' = dt iF and s the neighbours' sum: the
 // reference's step (TWMCBaseSolver.cpp:245-253) with dt folded into the
 // coefficients of the increment, whose terms are accumulated by multiply-adds
-// and added to b once.
+// and added to b once. HOP false: no such neighbours (s is not read).
+template <bool HOP = true>
 __device__ __forceinline__ Pair pair_update(Pair v, float2 sx, float2 sy, float2 ax, float2 ay, float2 bx, float2 by,
                                             float2 fx, float2 fy, float2 jt, const PairNoise& n) {
   const float2 ab2 = __ffma2_rn(v.y, v.y, __fmul2_rn(v.x, v.x));
   const float2 cx = __ffma2_rn(bx, ab2, ax), cy = __ffma2_rn(by, ab2, ay);
   float2 ix = __ffma2_rn(n.r, n.c, fx), iy = __ffma2_rn(n.r, n.s, fy);
-  ix = __ffma2_rn(jt, sy, ix);
-  iy = __ffma2_rn(neg2(jt), sx, iy);
+  if constexpr (HOP) {
+    ix = __ffma2_rn(jt, sy, ix);
+    iy = __ffma2_rn(neg2(jt), sx, iy);
+  }
   ix = __ffma2_rn(cx, v.x, ix);
   iy = __ffma2_rn(cx, v.y, iy);
   ix = __ffma2_rn(neg2(cy), v.y, ix);

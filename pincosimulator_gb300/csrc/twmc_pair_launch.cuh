@@ -92,4 +92,9 @@ bool pair_plan(const StepArgs& a, PairPlan* p);
 // Launches it (plan from pair_plan; a.tpt is taken from the plan).
 bool pair_launch(const StepArgs& a, const PairPlan& p, cudaStream_t s, LaunchInfo* info, std::string* err);
 
+// The packed Lieb kernel (twmc_lieb_pair.cu) for the same kind of run, F(t)
+// allowed: an even number of cells, at most 1024.
+bool lieb_pair_ok(const StepArgs& a);
+bool lieb_pair_launch(const StepArgs& a, cudaStream_t s, LaunchInfo* info, std::string* err);
+
 }  // namespace twmc

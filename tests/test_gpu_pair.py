@@ -63,3 +63,34 @@ def test_packed_bits_do_not_depend_on_the_batch(built_lib, shape):
     seeds = list(range(50, 50 + many))
     out = [run(nx, ny, "rsl", k, 20, beta0, seeds, np.random.default_rng(8))[0] for k in (1, 17, many)]
     assert np.array_equal(out[0], out[2][:1]) and np.array_equal(out[1], out[2][:17])
+
+
+@pytest.mark.parametrize("par,ramp", [("scalar", False), ("im", False), ("im", True), ("site", True), ("site", False)])
+@pytest.mark.parametrize("cells,pbc", [(2, True), (2, False), (6, True), (66, False), (256, True), (1024, False)])
+def test_packed_lieb_matches_oracle(built_lib, oracle, cells, pbc, par, ramp):
+    """The packed Lieb kernel (cells c and c + Nc/2 in the lanes): rings and
+    open chains, one slot to the most a CTA holds, F(t) over several table
+    segments, J_AB != J_BC so that each coupling lands on its bond."""
+    n, steps, dt = 3 * cells, 60, 0.002
+    rng = np.random.default_rng(cells)
+    beta0 = 0.4 * (rng.normal(size=(2, n)) + 1j * rng.normal(size=(2, n)))
+    E, U, F, F_t = 0.1, 0.27, 0.3, None
+    if par != "scalar":
+        E, U = 0.1 * rng.normal(size=n), 0.27 + 0.06 * rng.random(size=n)
+    if par == "site":
+        E, U, F = E + 0.02j * rng.normal(size=n), U + 0.01j * rng.normal(size=n), 0.3 + 0.1j * rng.normal(size=n)
+    if ramp:
+        times = np.round(np.arange(0, 0.09, 0.01), 10)
+        F_t = (times, np.outer(times / 0.05, 1.0 + 0.2 * rng.random(n)) * (1 + 0.3j))
+    s = twmc.System(lattice=twmc.LATTICE_LIEB, nx=1, ny=cells, pbc=pbc, J_AB=0.8, J_BC=1.3, gamma=1.0, detuning=0.5,
+                    dt=dt, frame_steps=steps, omega=E, U=U, F=F, F_t=F_t)
+    seeds = [7, 123]
+    tasks = s.make_tasks(2, t_end=steps * dt, ic=twmc.IC_GIVEN, init_field=beta0, seeds=seeds, id0=4)
+    res = s.run(tasks, frames=False)
+    assert s.kernel_name == "lieb_cell_kernel"
+    s.close()
+    for k in range(2):
+        xi = twmc.debug_wiener(twmc.PREC_F32, seeds[k], 4 + k, steps, n)
+        ref = oracle.lieb_run(cells, pbc, 0.8, 1.3, 0.5, 1.0, dt, 0.0, steps * dt, steps, 2, True, E, U, F, beta0[k],
+                              xi=xi, F_t=F_t)
+        assert rel_err(res["final"][k], ref["final"]) < 1e-5
