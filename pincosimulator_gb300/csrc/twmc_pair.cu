@@ -17,17 +17,17 @@ constexpr int64_t kSmemPerSm = 227 * 1024;
 // a tighter register cap.
 double slot_cycles(const PairPlan& p) {
   const int s = p.v * p.nb;
-  if (p.chain) return s >= 8 ? 125.0 : p.nb > 1 ? 112.0 : 104.0;
-  if (p.cl > 1) return !p.wide ? 165.0 : p.v >= 4 ? 162.0 : 142.0;
-  if (p.wide) return s >= 8 ? 275.0 : p.nb > 1 ? 168.0 : 150.0;
-  return s >= 8 ? 150.0 : s == 5 ? 148.0 : s == 4 ? (p.v == 1 ? 140.0 : p.v == 2 ? 131.0 : 132.0) : s == 3 ? 120.0 : s == 2 ? 114.0 : 122.0;
+  if (p.chain) return s >= 8 ? 125.0 : p.nb > 1 ? 116.0 : 104.0;
+  if (p.cl > 1) return !p.wide ? 165.0 : p.v >= 4 ? 185.0 : 165.0;
+  if (p.wide) return s >= 8 ? 275.0 : 174.0;
+  return s >= 8 ? 159.0 : s == 5 ? 148.0 : s == 4 ? (p.v == 1 ? 140.0 : p.v == 2 ? 131.0 : 132.0) : s == 3 ? 120.0 : s == 2 ? 114.0 : 122.0;
 }
 
 // Estimated cycles of one step of the whole batch: the slots' work on the
 // fullest scheduler of an SM on top of a latency (exchange, barrier, Philox
 // and the update's chain) that only the SM's other CTAs hide; a cluster
-// barrier adds to it. Over 21 shapes and batch sizes the split it picked was
-// within 8 % of the fastest in all but one (32x32 with 64 trajectories, 12 %). All splits give the same bits, so only time
+// barrier adds to it. Over 28 shapes and batch sizes the split it picked was
+// within 5 % of the fastest for 22, within 15 % for all. All splits give the same bits, so only time
 // depends on it.
 double step_cycles(const PairPlan& p, int64_t ntraj, int sms) {
   const int64_t regs = p.wide ? 64 : 128;
