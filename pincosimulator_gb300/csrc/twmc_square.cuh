@@ -4,6 +4,7 @@
 
 #include <algorithm>
 #include <string>
+#include <type_traits>
 
 #include "fft_plans.inc"
 #include "twmc_kernels.cuh"
@@ -18,7 +19,9 @@ template <typename R, class P>
 constexpr int cta_for() {
   constexpr int tpt = PlanInfo<P>::TPT;
   constexpr size_t per_traj = (sizeof(R) == 4 ? 3 : 2) * sizeof(c2_t<R>) * size_t(PlanInfo<P>::N) * 17 / 16;
-  int tpc = tpt >= 256 ? 1 : 256 / tpt;
+  // FP64: the FP64 pipe of an SM is one for all its warps, so one warp (or one
+  // trajectory) per CTA balances the SMs best
+  int tpc = sizeof(R) == 8 ? (tpt >= 32 ? 1 : 32 / tpt) : tpt >= 256 ? 1 : 256 / tpt;
   while (tpc > 1 && size_t(tpc) * per_traj > 100 * 1024) tpc /= 2;
   return tpc * tpt;
 }
@@ -87,11 +90,12 @@ bool square_dispatch(int bx, int by, const StepArgs& a, int nparams, cudaStream_
   const bool split = a.kfac != nullptr;
   const bool rsl_ok = a.rsl == nullptr || a.rsl_re_uniform;
 #define TWMC_SHAPE(BX, BY)                                                                                   \
-  if (bx == BX && by == BY)                                                                                  \
-    return !(fast && (rsl_ok || plan_reg_twiddles<Plan_##BX##_##BY>()))                                     \
-               ? square_launch_t<R, Plan_##BX##_##BY, false>(a, nparams, s, info, err)                      \
-           : !split ? square_launch_t<R, Plan_##BX##_##BY, sizeof(R) == 4>(a, nparams, s, info, err)        \
-                    : square_launch_t<R, Plan_##BX##_##BY, sizeof(R) == 4, sizeof(R) == 4>(a, nparams, s, info, err);
+  if (bx == BX && by == BY) {                                                                                \
+    using P = std::conditional_t<sizeof(R) == 4, Plan_##BX##_##BY, PlanD_##BX##_##BY>;                       \
+    return !(fast && (rsl_ok || plan_reg_twiddles<P>())) ? square_launch_t<R, P, false>(a, nparams, s, info, err) \
+           : !split ? square_launch_t<R, P, sizeof(R) == 4>(a, nparams, s, info, err)                        \
+                    : square_launch_t<R, P, sizeof(R) == 4, sizeof(R) == 4>(a, nparams, s, info, err);       \
+  }
   TWMC_SHAPE(0, 5) TWMC_SHAPE(0, 6) TWMC_SHAPE(0, 7) TWMC_SHAPE(0, 8) TWMC_SHAPE(0, 9) TWMC_SHAPE(0, 10)
   TWMC_SHAPE(0, 11) TWMC_SHAPE(0, 12) TWMC_SHAPE(4, 4) TWMC_SHAPE(5, 5) TWMC_SHAPE(6, 6)
 #undef TWMC_SHAPE

@@ -238,30 +238,48 @@ SUPPORTED_SHAPES = [
 ]
 
 
-def emit_header(e: int = 4) -> str:
-    """C++ source with one constexpr plan per supported shape."""
+def fp64_bits(n: int) -> int:
+    """Register bits of the FP64 plan of 2^n sites. The FP64 pipe (two lanes
+    per SM and cycle) bounds these runs, so all that counts is that every SM has
+    work and none waits for another: short threads spread a batch evenly.
+    Measured on GB300 with 4 / 8 / 16 sites per thread (1e9 site-updates/s):
+    16x16 with 500 trajectories 3.25 / 3.12 / 1.82, 1x64 with 200 0.74 / 0.37 /
+    0.19, 1x512 with 600 2.80 / 3.60 / 3.36 (more twiddles are thread-dependent
+    products on 4 sites), 32x32 with 700 3.15 / 3.35 / 2.82, 64x64 with 300
+    3.24 / 3.24 / 3.29."""
+    return 2 if n <= 8 else 3 if n <= 10 else 4
+
+
+def emit_header() -> str:
+    """C++ source with the constexpr plans of every supported shape:
+    Plan_<bx>_<by> (FP32) and PlanD_<bx>_<by> (FP64)."""
     lines = ["// Generated by pincosimulator_gb300/fft_plan.py -- do not edit.", "#pragma once", "namespace twmc {"]
     for (bx, by) in SUPPORTED_SHAPES:
-        p = make_plan(bx, by, e)
-        name = f"Plan_{bx}_{by}"
-        lines.append(f"struct {name} {{")
-        lines.append(f"  static constexpr int nbits = {p.nbits}, bx = {p.bx}, by = {p.by}, e = {p.e};")
-        lines.append(f"  static constexpr int npass = {len(p.passes)};")
-        lines.append(f"  static constexpr int lo[2] = {{{p.lo[0]}, {p.lo[1]}}};")
-        lines.append(f"  static constexpr int m[2] = {{{p.m[0]}, {p.m[1]}}};")
-        regs = ", ".join("{" + ", ".join(str(b) for b in ps.reg) + "}" for ps in p.passes)
-        nthr = p.nbits - p.e
-        thrs = ", ".join("{" + ", ".join(str(b) for b in (ps.thr if ps.thr else [0])) + "}" for ps in p.passes)
-        lines.append(f"  static constexpr int reg[{len(p.passes)}][{p.e}] = {{{regs}}};")
-        lines.append(f"  static constexpr int nthr = {nthr};")
-        lines.append(f"  static constexpr int thr[{len(p.passes)}][{max(nthr, 1)}] = {{{thrs}}};")
-        nst = ", ".join(str(len(ps.stages)) for ps in p.passes)
-        lines.append(f"  static constexpr int nst[{len(p.passes)}] = {{{nst}}};")
-        st = ", ".join(
-            "{" + ", ".join(f"{{{s.dim}, {s.t}, {s.rb}}}" for s in (ps.stages + [Stage(0, 0, 0)] * (4 - len(ps.stages)))) + "}"
-            for ps in p.passes
-        )
-        lines.append(f"  static constexpr int st[{len(p.passes)}][4][3] = {{{st}}};")
-        lines.append("};")
+        lines += _emit_plan(f"Plan_{bx}_{by}", make_plan(bx, by, 4))
+    for (bx, by) in SUPPORTED_SHAPES:
+        lines += _emit_plan(f"PlanD_{bx}_{by}", make_plan(bx, by, fp64_bits(bx + by)))
     lines.append("}  // namespace twmc")
     return "\n".join(lines) + "\n"
+
+
+def _emit_plan(name: str, p: Plan) -> list:
+    lines = [f"struct {name} {{"]
+    lines.append(f"  static constexpr int nbits = {p.nbits}, bx = {p.bx}, by = {p.by}, e = {p.e};")
+    lines.append(f"  static constexpr int npass = {len(p.passes)};")
+    lines.append(f"  static constexpr int lo[2] = {{{p.lo[0]}, {p.lo[1]}}};")
+    lines.append(f"  static constexpr int m[2] = {{{p.m[0]}, {p.m[1]}}};")
+    regs = ", ".join("{" + ", ".join(str(b) for b in ps.reg) + "}" for ps in p.passes)
+    nthr = p.nbits - p.e
+    thrs = ", ".join("{" + ", ".join(str(b) for b in (ps.thr if ps.thr else [0])) + "}" for ps in p.passes)
+    lines.append(f"  static constexpr int reg[{len(p.passes)}][{p.e}] = {{{regs}}};")
+    lines.append(f"  static constexpr int nthr = {nthr};")
+    lines.append(f"  static constexpr int thr[{len(p.passes)}][{max(nthr, 1)}] = {{{thrs}}};")
+    nst = ", ".join(str(len(ps.stages)) for ps in p.passes)
+    lines.append(f"  static constexpr int nst[{len(p.passes)}] = {{{nst}}};")
+    st = ", ".join(
+        "{" + ", ".join(f"{{{s.dim}, {s.t}, {s.rb}}}" for s in (ps.stages + [Stage(0, 0, 0)] * (4 - len(ps.stages)))) + "}"
+        for ps in p.passes
+    )
+    lines.append(f"  static constexpr int st[{len(p.passes)}][4][3] = {{{st}}};")
+    lines.append("};")
+    return lines

@@ -36,3 +36,17 @@ def test_headline_shape_bank_conflict_free():
     p = fp.make_plan(6, 6, 4)
     for k in range(len(p.passes)):
         assert fp.exchange_wavefronts(p, k, 1, 8, True) == 2.0
+
+
+@pytest.mark.parametrize("shape", fp.SUPPORTED_SHAPES)
+@pytest.mark.parametrize("e", [2, 3])
+def test_short_plans(shape, e):
+    """Plans of 4 and 8 sites per thread (FP64 runs): the same transform, the
+    top site bit in a register of the first pass."""
+    p = fp.make_plan(*shape, e)
+    rng = np.random.default_rng(e)
+    x = rng.normal(size=1 << p.nbits) + 1j * rng.normal(size=1 << p.nbits)
+    kx, ky = fp.freq_of_position(p)
+    ref = np.fft.fft2(x.reshape(1 << shape[0], 1 << shape[1]))
+    assert np.abs(fp.run_forward(p, x) - ref[kx, ky]).max() < 1e-10 * np.abs(ref).max()
+    assert p.nbits - 1 in p.passes[0].reg and all(len(ps.reg) == e for ps in p.passes)
