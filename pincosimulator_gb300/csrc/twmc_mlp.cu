@@ -9,13 +9,16 @@
 //   a BF16 copy of the same array feeds the GEMMs; gradients, Adam moments
 //   use the same offsets.
 //   Activations are BF16 (the GEMM operands), pre-activations FP32.
-// Every GEMM is one templated kernel: a 64 x 64 output tile per 128-thread
-// CTA, operands staged through shared memory with arbitrary strides (so the
-// transposed products of the backward pass need no transposed copies), and
-// mma.sync m16n8k16 BF16 x BF16 -> FP32 per warp on a 32 x 32 sub-tile.
-// The epilogue is fused: bias + GELU (hidden forward, keeping the FP32
-// pre-activation), bias (output layer), GELU' (backward), or plain store
-// (weight gradients).
+// Operands live in buffers of the network's own, rows padded to 16 bytes, so
+// that every tile load is a run of 16-byte asynchronous copies whatever the
+// widths. One kernel does every product (mma.sync m16n8k16 BF16 x BF16 ->
+// FP32): tiles of 64 x 64, or 32 x 32 where those would be too few for the
+// SMs, four stages of operands in flight, either operand row-major along K or
+// along its rows (ldmatrix transposes), and the epilogue fused: bias + GELU
+// (hidden forward, keeping the FP32 pre-activation), bias (output layer), bias
+// + MSE gradient and loss (output layer of a backward call), GELU' (backward),
+// weight gradients with the bias gradients' column sums. A backward layer's
+// two products are one launch.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -32,22 +35,36 @@ namespace {
 
 using bf16 = __nv_bfloat16;
 
-constexpr int kBM = 64, kBN = 64, kBK = 32, kPadK = kBK + 8;
+constexpr int kStages = 4;
 
-enum Epi { EPI_BIAS_GELU = 0, EPI_BIAS = 1, EPI_GELU_BWD = 2, EPI_STORE = 3 };
+enum Epi { EPI_BIAS_GELU = 0, EPI_BIAS = 1, EPI_GELU_BWD = 2, EPI_DW = 3, EPI_MSE = 4 };
 
-// C[m][n] = sum_k A(m, k) B(n, k), A(m, k) = A[m sam + k sak], B(n, k) = B[n sbn + k sbk].
+// C[m][n] = sum_k A(m, k) B(n, k). An operand is stored [row][k] (kmajor) or
+// [k][row], ld elements apart (a multiple of 8, base 16-byte aligned).
 struct GemmArgs {
   const bf16* A;
-  int64_t sam, sak;
+  int64_t lda;
+  int a_kmajor;
   const bf16* B;
-  int64_t sbn, sbk;
+  int64_t ldb;
+  int b_kmajor;
   int M, N, K;
-  const float* bias;  // [N]            (EPI_BIAS_GELU, EPI_BIAS)
-  const float* z;     // [M][ldo] FP32  (EPI_GELU_BWD)
-  float* outf;        // [M][ldo] FP32  (EPI_BIAS_GELU: z, EPI_BIAS, EPI_STORE)
-  bf16* outh;         // [M][ldo] BF16  (EPI_BIAS_GELU: gelu(z), EPI_GELU_BWD)
-  int64_t ldo;
+  int epi;
+  const float* bias;    // [N]            (EPI_BIAS_GELU, EPI_BIAS, EPI_MSE)
+  const float* z;       // [M][ldf] FP32  (EPI_GELU_BWD)
+  float* outf;          // [M][ldf] FP32  (EPI_BIAS_GELU: z, EPI_BIAS, EPI_DW)
+  int64_t ldf;
+  bf16* outh;           // [M][ldh] BF16  (EPI_BIAS_GELU: gelu(z), EPI_GELU_BWD, EPI_MSE: the loss gradient)
+  int64_t ldh;
+  float* colsum;        // [M] sums of A over k (EPI_DW: the bias gradients)
+  const float* target;  // [M][N]         (EPI_MSE)
+  const float* weight;  // [N] or NULL    (EPI_MSE)
+  float* loss;          // (EPI_MSE)
+  int tiles_n, tiles;
+};
+// Up to two products in one launch: CTAs [0, first.tiles) do the first.
+struct GemmPair {
+  GemmArgs g[2];
 };
 
 __device__ __forceinline__ float gelu_f(float z) { return 0.5f * z * (1.0f + erff(z * 0.70710678118654752f)); }
@@ -65,143 +82,261 @@ __device__ __forceinline__ void mma_bf16_16816(float (&d)[4], const uint32_t (&a
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 
-// Stages a rows x kBK tile (row r0.., k k0..) into s[row][k], zero outside.
-// Consecutive threads walk the unit-stride dimension of the source.
-__device__ __forceinline__ void stage_tile(bf16 (*s)[kPadK], const bf16* src, int64_t sr, int64_t sk, int nrows,
-                                           int nk, int r0, int k0) {
-  const bf16 zero = __float2bfloat16(0.0f);
-  for (int i = threadIdx.x; i < kBM * kBK; i += blockDim.x) {
-    int r, c;
-    if (sk == 1) { r = i / kBK; c = i % kBK; }
-    else { r = i % kBM; c = i / kBM; }
-    const int gr = r0 + r, gk = k0 + c;
-    s[r][c] = (gr < nrows && gk < nk) ? src[int64_t(gr) * sr + int64_t(gk) * sk] : zero;
-  }
+__device__ __forceinline__ uint32_t sm_addr(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
+// 16 bytes from global to shared memory, `valid` of them read and the rest zero.
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, int valid) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid) : "memory");
+}
+__device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], uint32_t a) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
+}
+__device__ __forceinline__ void ldmatrix4_trans(uint32_t (&r)[4], uint32_t a) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
 }
 
-template <int EPI>
-__global__ void __launch_bounds__(128) mlp_gemm_kernel(const GemmArgs g) {
-  __shared__ __align__(16) bf16 As[kBM][kPadK];
-  __shared__ __align__(16) bf16 Bs[kBN][kPadK];
+// Bytes between consecutive lines of a tile: [R][BK] (kmajor) or [BK][R], 16
+// bytes of padding so that the eight lines of an ldmatrix hit all banks.
+template <int R, int BK> __device__ __forceinline__ constexpr int tile_pitch(bool kmajor) { return (kmajor ? BK : R) * 2 + 16; }
+template <int R, int BK> constexpr int tile_bytes() {
+  constexpr int a = R * (BK * 2 + 16), b = BK * (R * 2 + 16);
+  return a > b ? a : b;
+}
+
+// One thread's share of an operand's R x BK tiles: kChunks pieces of 16 bytes,
+// whose sources advance by one tile of k per call. Out of range is zero.
+template <int R, int BK> struct TileLoader {
+  static constexpr int kChunks = R * BK / 8 / 128;
+  static_assert(R * BK % (8 * 128) == 0, "whole chunks per thread");
+  const bf16* base;
+  const bf16* src[kChunks];
+  int dst[kChunks];
+  int a[kChunks], b[kChunks];  // kmajor: elements left in the line (0: no such line); else lines left, elements in the line
+  int64_t advance;
+  bool kmajor;
+  __device__ __forceinline__ TileLoader(const bf16* p, int64_t ld, bool km, int rows, int K, int r0) : base(p), kmajor(km) {
+    advance = km ? BK : BK * ld;
+#pragma unroll
+    for (int i = 0; i < kChunks; ++i) {
+      const int id = threadIdx.x + i * 128;
+      const int line = km ? id / (BK / 8) : id / (R / 8), c = (km ? id % (BK / 8) : id % (R / 8)) * 8;
+      dst[i] = line * tile_pitch<R, BK>(km) + c * 2;
+      if (km) {
+        src[i] = p + int64_t(r0 + line) * ld + c;
+        a[i] = r0 + line < rows ? K - c : 0;
+        b[i] = 0;
+      } else {
+        src[i] = p + int64_t(line) * ld + r0 + c;
+        a[i] = K - line;
+        b[i] = min(max(rows - (r0 + c), 0), 8);
+      }
+    }
+  }
+  __device__ __forceinline__ void load(uint32_t tile) {
+#pragma unroll
+    for (int i = 0; i < kChunks; ++i) {
+      const int valid = kmajor ? min(max(a[i], 0), 8) : a[i] > 0 ? b[i] : 0;
+      cp_async16(tile + uint32_t(dst[i]), valid ? src[i] : base, valid * 2);
+      src[i] += advance;
+      a[i] -= BK;
+    }
+  }
+};
+
+// What bounds a training step is latency: its products are 0.03 to 0.3 GFLOP, one
+// after the other. Hence small tiles on many SMs, four stages of copies ahead
+// of the tensor cores, and few launches. Measured on GB300 (5-256-256-256-2049,
+// 128 rows): 660 us per step with two-byte loads, no copies ahead and 17
+// launches, 72 us in this form with 10.
+// The k16 products of an output are accumulated in ascending order, so
+// the results do not depend on the tile.
+template <int BM, int BN, int BK>
+__global__ void __launch_bounds__(128) mlp_gemm_kernel(const __grid_constant__ GemmPair pair) {
+  __shared__ __align__(16) unsigned char sA[kStages][tile_bytes<BM, BK>()];
+  __shared__ __align__(16) unsigned char sB[kStages][tile_bytes<BN, BK>()];
+  const bool second = int(blockIdx.x) >= pair.g[0].tiles;
+  const GemmArgs& g = pair.g[second ? 1 : 0];
+  const int tile = int(blockIdx.x) - (second ? pair.g[0].tiles : 0);
+  const int m0 = (tile / g.tiles_n) * BM, n0 = (tile % g.tiles_n) * BN;
+  const bool ak = g.a_kmajor != 0, bk = g.b_kmajor != 0;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int gq = lane >> 2, tq = lane & 3;
-  const int m0 = blockIdx.y * kBM, n0 = blockIdx.x * kBN;
-  const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
-  float acc[2][4][4];
+  constexpr int MI = BM / 32, NI = BN / 16;  // 16-row and 8-column blocks of a warp (2 x 2 warps)
+  const int wm = (warp >> 1) * (BM / 2), wn = (warp & 1) * (BN / 2);
+  const int pa = tile_pitch<BM, BK>(ak), pb = tile_pitch<BN, BK>(bk);
+  // ldmatrix source of this lane in an operand block (see the two layouts)
+  const int mi = lane >> 3, r8 = lane & 7;
+  const int a_off = ak ? (wm + (mi & 1) * 8 + r8) * pa + (mi >> 1) * 16 : ((mi >> 1) * 8 + r8) * pa + (wm + (mi & 1) * 8) * 2;
+  const int b_off = bk ? (wn + (mi >> 1) * 8 + r8) * pb + (mi & 1) * 16 : ((mi & 1) * 8 + r8) * pb + (wn + (mi >> 1) * 8) * 2;
+  float acc[MI][NI][4];
 #pragma unroll
-  for (int i = 0; i < 2; ++i)
+  for (int i = 0; i < MI; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
+    for (int j = 0; j < NI; ++j)
 #pragma unroll
       for (int c = 0; c < 4; ++c) acc[i][j][c] = 0.0f;
-  for (int k0 = 0; k0 < g.K; k0 += kBK) {
-    stage_tile(As, g.A, g.sam, g.sak, g.M, g.K, m0, k0);
-    stage_tile(Bs, g.B, g.sbn, g.sbk, g.N, g.K, n0, k0);
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < kBK; kk += 16) {
-      uint32_t af[2][4], bfr[4][2];
-#pragma unroll
-      for (int mi = 0; mi < 2; ++mi) {
-        const int r = wm + mi * 16 + gq;
-        af[mi][0] = *reinterpret_cast<const uint32_t*>(&As[r][kk + 2 * tq]);
-        af[mi][1] = *reinterpret_cast<const uint32_t*>(&As[r + 8][kk + 2 * tq]);
-        af[mi][2] = *reinterpret_cast<const uint32_t*>(&As[r][kk + 2 * tq + 8]);
-        af[mi][3] = *reinterpret_cast<const uint32_t*>(&As[r + 8][kk + 2 * tq + 8]);
-      }
-#pragma unroll
-      for (int ni = 0; ni < 4; ++ni) {
-        const int c = wn + ni * 8 + gq;
-        bfr[ni][0] = *reinterpret_cast<const uint32_t*>(&Bs[c][kk + 2 * tq]);
-        bfr[ni][1] = *reinterpret_cast<const uint32_t*>(&Bs[c][kk + 2 * tq + 8]);
-      }
-#pragma unroll
-      for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-        for (int ni = 0; ni < 4; ++ni) mma_bf16_16816(acc[mi][ni], af[mi], bfr[ni]);
+  const int steps = (g.K + BK - 1) / BK;
+  TileLoader<BM, BK> la(g.A, g.lda, ak, g.M, g.K, m0);
+  TileLoader<BN, BK> lb(g.B, g.ldb, bk, g.N, g.K, n0);
+  auto fetch = [&](int s) {
+    if (s < steps) {
+      la.load(sm_addr(sA[s % kStages]));
+      lb.load(sm_addr(sB[s % kStages]));
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int s = 0; s < kStages - 1; ++s) fetch(s);
+  // column sums of A over k, ascending (the bias gradients), by the CTAs of the first column of tiles
+  const bool sums = g.epi == EPI_DW && n0 == 0 && int(threadIdx.x) < BM;
+  float csum = 0.0f;
+  for (int s = 0; s < steps; ++s) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
     __syncthreads();
+    fetch(s + kStages - 1);  // into the stage that the barrier has freed
+    const uint32_t ta = sm_addr(sA[s % kStages]), tb = sm_addr(sB[s % kStages]);
+#pragma unroll
+    for (int kk = 0; kk < BK; kk += 16) {
+      uint32_t af[MI][4], bfr[NI / 2][4];
+#pragma unroll
+      for (int i = 0; i < MI; ++i) {
+        if (ak) ldmatrix4(af[i], ta + uint32_t(a_off + i * 16 * pa + kk * 2));
+        else ldmatrix4_trans(af[i], ta + uint32_t(a_off + i * 32 + kk * pa));
+      }
+#pragma unroll
+      for (int j = 0; j < NI / 2; ++j) {
+        if (bk) ldmatrix4(bfr[j], tb + uint32_t(b_off + j * 16 * pb + kk * 2));
+        else ldmatrix4_trans(bfr[j], tb + uint32_t(b_off + j * 32 + kk * pb));
+      }
+#pragma unroll
+      for (int i = 0; i < MI; ++i)
+#pragma unroll
+        for (int j = 0; j < NI; ++j) {
+          const uint32_t b2[2] = {bfr[j / 2][(j & 1) * 2], bfr[j / 2][(j & 1) * 2 + 1]};
+          mma_bf16_16816(acc[i][j], af[i], b2);
+        }
+    }
+    if (sums) {
+#pragma unroll 8
+      for (int k = 0; k < BK; ++k)
+        csum += __bfloat162float(*reinterpret_cast<const bf16*>(
+            sA[s % kStages] + (ak ? threadIdx.x * pa + k * 2 : k * pa + threadIdx.x * 2)));
+    }
   }
+  if (sums && m0 + int(threadIdx.x) < g.M) g.colsum[m0 + threadIdx.x] = csum;
+  float part = 0.0f;
+  const float inv = 1.0f / float(int64_t(g.M) * g.N);
 #pragma unroll
-  for (int mi = 0; mi < 2; ++mi)
+  for (int i = 0; i < MI; ++i)
 #pragma unroll
-    for (int ni = 0; ni < 4; ++ni)
+    for (int j = 0; j < NI; ++j)
 #pragma unroll
       for (int h = 0; h < 2; ++h)
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
-          const int row = m0 + wm + mi * 16 + gq + 8 * h;
-          const int col = n0 + wn + ni * 8 + 2 * tq + c;
+          const int row = m0 + wm + i * 16 + gq + 8 * h;
+          const int col = n0 + wn + j * 8 + 2 * tq + c;
           if (row >= g.M || col >= g.N) continue;
-          const float v = acc[mi][ni][2 * h + c];
-          const int64_t idx = int64_t(row) * g.ldo + col;
-          if constexpr (EPI == EPI_BIAS_GELU) {
+          const float v = acc[i][j][2 * h + c];
+          const int64_t fi = int64_t(row) * g.ldf + col, hi = int64_t(row) * g.ldh + col;
+          if (g.epi == EPI_BIAS_GELU) {
             const float z = v + g.bias[col];
-            g.outf[idx] = z;
-            g.outh[idx] = __float2bfloat16(gelu_f(z));
-          } else if constexpr (EPI == EPI_BIAS) {
-            g.outf[idx] = v + g.bias[col];
-          } else if constexpr (EPI == EPI_GELU_BWD) {
-            g.outh[idx] = __float2bfloat16(v * gelu_grad(g.z[idx]));
-          } else {
-            g.outf[idx] = v;
+            g.outf[fi] = z;
+            g.outh[hi] = __float2bfloat16(gelu_f(z));
+          } else if (g.epi == EPI_BIAS) {
+            g.outf[fi] = v + g.bias[col];
+          } else if (g.epi == EPI_GELU_BWD) {
+            g.outh[hi] = __float2bfloat16(v * gelu_grad(g.z[fi]));
+          } else if (g.epi == EPI_DW) {
+            g.outf[fi] = v;
+          } else {  // dy = bf16(2 w_o (y - t) / (M O)); loss += sum w_o (y - t)^2 / (M O)
+            const float wo = g.weight ? g.weight[col] : 1.0f;
+            const float e = (v + g.bias[col]) - g.target[int64_t(row) * g.N + col];
+            part += wo * e * e;
+            g.outh[hi] = __float2bfloat16(2.0f * wo * e * inv);
           }
         }
-}
-
-__global__ void cast_bf16_kernel(const float* __restrict__ x, int64_t n, bf16* __restrict__ y) {
-  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
-    y[i] = __float2bfloat16(x[i]);
-}
-
-// dy = bf16(2 w_o (y - t) / (M O)); *loss += sum w_o (y - t)^2 / (M O).
-__global__ void mse_grad_kernel(const float* __restrict__ y, const float* __restrict__ t,
-                                const float* __restrict__ w, int64_t M, int O, bf16* __restrict__ dy,
-                                float* __restrict__ loss) {
-  const int64_t n = M * O;
-  const float inv = 1.0f / float(n);
-  float part = 0.0f;
-  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
-    const float wo = w ? w[i % O] : 1.0f;
-    const float e = y[i] - t[i];
-    part += wo * e * e;
-    dy[i] = __float2bfloat16(2.0f * wo * e * inv);
-  }
+  if (g.epi == EPI_MSE) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-  __shared__ float red[32];
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = part;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float s = 0.0f;
-    for (int i = 0; i < int(blockDim.x >> 5); ++i) s += red[i];
-    atomicAdd(loss, s * inv);
+    for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+    __shared__ float red[4];
+    if (lane == 0) red[warp] = part;
+    __syncthreads();
+    if (threadIdx.x == 0) atomicAdd(g.loss, ((red[0] + red[1]) + (red[2] + red[3])) * inv);
   }
 }
 
-// out[n] = sum_m d[m][n] (FP32, sequential in m: deterministic).
-__global__ void colsum_kernel(const bf16* __restrict__ d, int64_t M, int N, float* __restrict__ out) {
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= N) return;
-  float s = 0.0f;
-  for (int64_t m = 0; m < M; ++m) s += __bfloat162float(d[m * N + n]);
-  out[n] = s;
+// BF16 copy of x [rows][cols] into y, ld apart; zeroes *loss (NULL: none).
+__global__ void cast_input_kernel(const float* __restrict__ x, int64_t rows, int cols, bf16* __restrict__ y, int64_t ld,
+                                  float* __restrict__ loss) {
+  if (loss && blockIdx.x == 0 && threadIdx.x == 0) *loss = 0.0f;
+  const int64_t n = rows * cols;
+  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
+    y[(i / cols) * ld + i % cols] = __float2bfloat16(x[i]);
 }
 
-// Adam (Kingma & Ba 2015) on the FP32 master copy; refreshes the BF16 copy.
-// c1 = 1 / (1 - beta1^t), c2 = 1 / (1 - beta2^t).
+// Where the layers' parameters lie: W_l [n][k] and then b_l [n] at `off` of the
+// FP32 arrays, the BF16 copy of W_l at `h`, ld apart.
+constexpr int kMaxLayers = 16;
+struct LayerMap {
+  int64_t off[kMaxLayers], h[kMaxLayers];
+  int n[kMaxLayers], k[kMaxLayers], ld[kMaxLayers];
+};
+
+// The BF16 copy of every layer's weights: grid (rows, layer).
+__global__ void cast_params_kernel(const float* __restrict__ w, bf16* __restrict__ w16, const __grid_constant__ LayerMap m) {
+  const int l = blockIdx.y, K = m.k[l];
+  for (int r = blockIdx.x; r < m.n[l]; r += gridDim.x)
+    for (int c = threadIdx.x; c < K; c += blockDim.x)
+      w16[m.h[l] + int64_t(r) * m.ld[l] + c] = __float2bfloat16(w[m.off[l] + int64_t(r) * K + c]);
+}
+
+// Adam (Kingma & Ba 2015) on the FP32 master copy, four parameters per thread;
+// refreshes the BF16 copy. c1 = 1 / (1 - beta1^t), c2 = 1 / (1 - beta2^t).
+__device__ __forceinline__ float adam_one(float w, float g, float& m, float& v, float lr, float b1, float b2, float eps,
+                                          float c1, float c2) {
+  m = b1 * m + (1.0f - b1) * g;
+  v = b2 * v + (1.0f - b2) * g * g;
+  return w - lr * (m * c1) / (sqrtf(v * c2) + eps);
+}
 __global__ void adam_kernel(float* __restrict__ w, bf16* __restrict__ w16, const float* __restrict__ g,
-                            float* __restrict__ m, float* __restrict__ v, int64_t n, float lr, float b1, float b2,
-                            float eps, float c1, float c2) {
-  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
-    const float gi = g[i];
-    const float mi = b1 * m[i] + (1.0f - b1) * gi;
-    const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    const float wi = w[i] - lr * (mi * c1) / (sqrtf(vi * c2) + eps);
-    w[i] = wi;
-    w16[i] = __float2bfloat16(wi);
+                            float* __restrict__ m, float* __restrict__ v, int64_t n, const __grid_constant__ LayerMap lm,
+                            int nl, float lr, float b1, float b2, float eps, float c1, float c2) {
+  for (int64_t i = 4 * (blockIdx.x * int64_t(blockDim.x) + threadIdx.x); i < n; i += 4 * int64_t(gridDim.x) * blockDim.x) {
+    float wv[4], gv[4], mv[4], vv[4];
+    const int cnt = int(min(int64_t(4), n - i));
+    if (cnt == 4) {
+      *reinterpret_cast<float4*>(wv) = *reinterpret_cast<const float4*>(w + i);
+      *reinterpret_cast<float4*>(gv) = *reinterpret_cast<const float4*>(g + i);
+      *reinterpret_cast<float4*>(mv) = *reinterpret_cast<const float4*>(m + i);
+      *reinterpret_cast<float4*>(vv) = *reinterpret_cast<const float4*>(v + i);
+    } else {
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        if (c < cnt) { wv[c] = w[i + c]; gv[c] = g[i + c]; mv[c] = m[i + c]; vv[c] = v[i + c]; }
+        else wv[c] = gv[c] = mv[c] = vv[c] = 0.0f;
+    }
+#pragma unroll
+    for (int c = 0; c < 4; ++c) wv[c] = adam_one(wv[c], gv[c], mv[c], vv[c], lr, b1, b2, eps, c1, c2);
+    if (cnt == 4) {
+      *reinterpret_cast<float4*>(w + i) = *reinterpret_cast<const float4*>(wv);
+      *reinterpret_cast<float4*>(m + i) = *reinterpret_cast<const float4*>(mv);
+      *reinterpret_cast<float4*>(v + i) = *reinterpret_cast<const float4*>(vv);
+    } else {
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        if (c < cnt) { w[i + c] = wv[c]; m[i + c] = mv[c]; v[i + c] = vv[c]; }
+    }
+    int l = 0;
+    while (l + 1 < nl && i >= lm.off[l + 1]) ++l;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      if (c >= cnt) break;
+      if (l + 1 < nl && i + c >= lm.off[l + 1]) ++l;
+      const uint32_t at = uint32_t(i + c - lm.off[l]), r = at / uint32_t(lm.k[l]);
+      if (r < uint32_t(lm.n[l])) w16[lm.h[l] + int64_t(r) * lm.ld[l] + (at - r * uint32_t(lm.k[l]))] = __float2bfloat16(wv[c]);
+    }
   }
 }
 
@@ -391,10 +526,10 @@ struct twmc_mlp {
   int max_width = 0;
   DevArr<float> w, g, m, v;
   DevArr<bf16> w16;
-  std::vector<DevArr<bf16>> act;  // act[l]: input of layer l, [max_batch][width[l]]
+  LayerMap map{};
+  std::vector<DevArr<bf16>> act;  // act[l]: input of layer l, [max_batch][pad8(width[l])]
   std::vector<DevArr<float>> z;   // z[l]: pre-activation output of layer l-1, [max_batch][width[l]] (l = 1..nl-1)
-  DevArr<float> y;                // [max_batch][width[nl]]
-  DevArr<bf16> d0, d1;            // backward ping-pong, [max_batch][max_width]
+  DevArr<bf16> d0, d1;            // backward ping-pong, [max_batch][pad8(width)]
   DevArr<float> loss;
   int64_t launches = 0;
   std::string err;
@@ -407,38 +542,66 @@ int mfail(twmc_mlp* m, int code, const std::string& s) {
   return code;
 }
 
-template <int EPI>
-bool gemm(twmc_mlp* m, const GemmArgs& g, cudaStream_t s) {
-  dim3 grid(unsigned((g.N + kBN - 1) / kBN), unsigned((g.M + kBM - 1) / kBM));
-  mlp_gemm_kernel<EPI><<<grid, 128, 0, s>>>(g);
+int64_t pad8(int64_t n) { return (n + 7) & ~int64_t(7); }
+
+// One launch of one product, or of two that depend on the same input: 64 x 64
+// tiles where they come to at least 96 CTAs and no sum is long, else 32 x 32
+// with 64 of K at a time (on 64 x 64 tiles a sum over 2049 ran on 8 CTAs, 47 us
+// of a training step's 119).
+bool gemm(twmc_mlp* m, GemmArgs a, cudaStream_t s, const GemmArgs* b = nullptr) {
+  GemmPair p{};
+  auto tiles = [](GemmArgs& g, int t) {
+    g.tiles_n = (g.N + t - 1) / t;
+    g.tiles = ((g.M + t - 1) / t) * g.tiles_n;
+    return int64_t(g.tiles);
+  };
+  p.g[0] = a;
+  if (b) p.g[1] = *b;
+  int64_t n = tiles(p.g[0], 64) + (b ? tiles(p.g[1], 64) : 0);
+  if (n >= 96 && std::max(p.g[0].K, p.g[1].K) <= 512) {
+    mlp_gemm_kernel<64, 64, 32><<<unsigned(n), 128, 0, s>>>(p);
+  } else {
+    n = tiles(p.g[0], 32) + (b ? tiles(p.g[1], 32) : 0);
+    mlp_gemm_kernel<32, 32, 64><<<unsigned(n), 128, 0, s>>>(p);
+  }
   ++m->launches;
   return cudaPeekAtLastError() == cudaSuccess;
 }
 
-// Forward pass of `batch` rows of x (device FP32 [batch][width[0]]) into y
-// (device FP32 [batch][width[nl]]), keeping activations for the backward.
-bool forward_chunk(twmc_mlp* m, const float* x, int64_t batch, float* yout, cudaStream_t s) {
+// Forward pass of `batch` rows of x (device FP32 [batch][width[0]]), keeping
+// activations for the backward. The output layer goes to yout (device FP32
+// [batch][width[nl]]), or, with a target, to the loss and its gradient (d0).
+bool forward_chunk(twmc_mlp* m, const float* x, int64_t batch, float* yout, cudaStream_t s,
+                   const float* target = nullptr, const float* weight = nullptr) {
   const int64_t nin = batch * m->width[0];
-  cast_bf16_kernel<<<grid_for(nin, 256), 256, 0, s>>>(x, nin, m->act[0].p);
+  cast_input_kernel<<<grid_for(nin, 256), 256, 0, s>>>(x, batch, m->width[0], m->act[0].p, pad8(m->width[0]),
+                                                       target ? m->loss.p : nullptr);
   ++m->launches;
   for (int l = 0; l < m->nl; ++l) {
     const int K = m->width[l], N = m->width[l + 1];
     GemmArgs g{};
-    g.A = m->act[l].p; g.sam = K; g.sak = 1;
-    g.B = m->w16.p + m->w_off[l]; g.sbn = K; g.sbk = 1;
+    g.A = m->act[l].p; g.lda = pad8(K); g.a_kmajor = 1;
+    g.B = m->w16.p + m->map.h[l]; g.ldb = m->map.ld[l]; g.b_kmajor = 1;
     g.M = int(batch); g.N = N; g.K = K;
     g.bias = m->w.p + m->b_off[l];
-    g.ldo = N;
-    bool ok;
+    g.ldf = N;
     if (l + 1 < m->nl) {
+      g.epi = EPI_BIAS_GELU;
       g.outf = m->z[l + 1].p;
       g.outh = m->act[l + 1].p;
-      ok = gemm<EPI_BIAS_GELU>(m, g, s);
+      g.ldh = pad8(N);
+    } else if (target) {
+      g.epi = EPI_MSE;
+      g.target = target;
+      g.weight = weight;
+      g.loss = m->loss.p;
+      g.outh = m->d0.p;
+      g.ldh = pad8(N);
     } else {
+      g.epi = EPI_BIAS;
       g.outf = yout;
-      ok = gemm<EPI_BIAS>(m, g, s);
     }
-    if (!ok) return false;
+    if (!gemm(m, g, s)) return false;
   }
   return true;
 }
@@ -473,14 +636,23 @@ int twmc_mlp_create(int32_t n_layers, const int32_t* widths, int64_t max_batch, 
     off += widths[l + 1];
   }
   m->nparam = off;
+  int64_t h = 0;
+  for (int l = 0; l < n_layers; ++l) {
+    m->map.off[l] = m->w_off[l];
+    m->map.n[l] = widths[l + 1];
+    m->map.k[l] = widths[l];
+    m->map.ld[l] = int(pad8(widths[l]));
+    m->map.h[l] = h;
+    h += int64_t(widths[l + 1]) * m->map.ld[l];
+  }
   m->max_width = *std::max_element(m->width.begin(), m->width.end());
   m->act.resize(n_layers);
   m->z.resize(n_layers);
-  bool ok = m->w.alloc(off) && m->g.alloc(off) && m->m.alloc(off) && m->v.alloc(off) && m->w16.alloc(off) &&
-            m->y.alloc(size_t(max_batch) * widths[n_layers]) && m->d0.alloc(size_t(max_batch) * m->max_width) &&
-            m->d1.alloc(size_t(max_batch) * m->max_width) && m->loss.alloc(1);
+  bool ok = m->w.alloc(off) && m->g.alloc(off) && m->m.alloc(off) && m->v.alloc(off) && m->w16.alloc(h) &&
+            m->d0.alloc(size_t(max_batch) * pad8(m->max_width)) && m->d1.alloc(size_t(max_batch) * pad8(m->max_width)) &&
+            m->loss.alloc(1);
   for (int l = 0; l < n_layers && ok; ++l) {
-    ok = m->act[l].alloc(size_t(max_batch) * widths[l]);
+    ok = m->act[l].alloc(size_t(max_batch) * pad8(widths[l]));
     if (ok && l > 0) ok = m->z[l].alloc(size_t(max_batch) * widths[l]);
   }
   if (!ok) {
@@ -510,7 +682,7 @@ int twmc_mlp_set_params(twmc_mlp* m, const float* host) {
       cudaMemset(m->m.p, 0, n * sizeof(float)) != cudaSuccess || cudaMemset(m->v.p, 0, n * sizeof(float)) != cudaSuccess ||
       cudaMemset(m->g.p, 0, n * sizeof(float)) != cudaSuccess)
     return mfail(m, TWMC_ERR_CUDA, "parameter upload failed");
-  cast_bf16_kernel<<<grid_for(int64_t(n), 256), 256>>>(m->w.p, int64_t(n), m->w16.p);
+  cast_params_kernel<<<dim3(unsigned(std::min(m->max_width, 4096)), unsigned(m->nl)), 256>>>(m->w.p, m->w16.p, m->map);
   ++m->launches;
   m->step = 0;
   const cudaError_t e = cudaDeviceSynchronize();
@@ -554,37 +726,36 @@ int twmc_mlp_backward(twmc_mlp* m, const float* x, const float* target, const fl
   if (!m || !x || !target || batch < 1 || batch > m->max_batch) return TWMC_ERR_INVALID;
   cudaSetDevice(m->device);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const int nl = m->nl, O = m->width[nl];
-  if (!forward_chunk(m, x, batch, m->y.p, s)) { cudaGetLastError(); return mfail(m, TWMC_ERR_CUDA, "forward launch failed"); }
-  cudaMemsetAsync(m->loss.p, 0, sizeof(float), s);
-  mse_grad_kernel<<<grid_for(batch * O, 256), 256, 0, s>>>(m->y.p, target, weights, batch, O, m->d0.p, m->loss.p);
-  ++m->launches;
+  if (!forward_chunk(m, x, batch, nullptr, s, target, weights)) { cudaGetLastError(); return mfail(m, TWMC_ERR_CUDA, "forward launch failed"); }
   bf16* dcur = m->d0.p;
   bf16* dnext = m->d1.p;
-  for (int l = nl - 1; l >= 0; --l) {
+  for (int l = m->nl - 1; l >= 0; --l) {
     const int K = m->width[l], N = m->width[l + 1];
-    // dW_l[n][k] = sum_b dZ[b][n] act_l[b][k]
+    // dW_l[n][k] = sum_b dZ[b][n] act_l[b][k], db_l[n] = sum_b dZ[b][n]
     GemmArgs gw{};
-    gw.A = dcur; gw.sam = 1; gw.sak = N;
-    gw.B = m->act[l].p; gw.sbn = 1; gw.sbk = K;
+    gw.A = dcur; gw.lda = pad8(N);
+    gw.B = m->act[l].p; gw.ldb = pad8(K);
     gw.M = N; gw.N = K; gw.K = int(batch);
+    gw.epi = EPI_DW;
     gw.outf = m->g.p + m->w_off[l];
-    gw.ldo = K;
-    if (!gemm<EPI_STORE>(m, gw, s)) { cudaGetLastError(); return mfail(m, TWMC_ERR_CUDA, "backward launch failed"); }
-    colsum_kernel<<<(N + 127) / 128, 128, 0, s>>>(dcur, batch, N, m->g.p + m->b_off[l]);
-    ++m->launches;
+    gw.ldf = K;
+    gw.colsum = m->g.p + m->b_off[l];
+    // dZ_{l-1}[b][k] = (sum_n dZ[b][n] W_l[n][k]) gelu'(z_l[b][k])
+    GemmArgs gd{};
     if (l > 0) {
-      // dZ_{l-1}[b][k] = (sum_n dZ[b][n] W_l[n][k]) gelu'(z_l[b][k])
-      GemmArgs gd{};
-      gd.A = dcur; gd.sam = N; gd.sak = 1;
-      gd.B = m->w16.p + m->w_off[l]; gd.sbn = 1; gd.sbk = K;
+      gd.A = dcur; gd.lda = pad8(N); gd.a_kmajor = 1;
+      gd.B = m->w16.p + m->map.h[l]; gd.ldb = m->map.ld[l];
       gd.M = int(batch); gd.N = K; gd.K = N;
+      gd.epi = EPI_GELU_BWD;
       gd.z = m->z[l].p;
+      gd.ldf = K;
       gd.outh = dnext;
-      gd.ldo = K;
-      if (!gemm<EPI_GELU_BWD>(m, gd, s)) { cudaGetLastError(); return mfail(m, TWMC_ERR_CUDA, "backward launch failed"); }
-      std::swap(dcur, dnext);
+      gd.ldh = pad8(K);
     }
+    // the longer sum's tiles first
+    const bool ok = l > 0 ? gemm(m, gd, s, &gw) : gemm(m, gw, s);
+    if (!ok) { cudaGetLastError(); return mfail(m, TWMC_ERR_CUDA, "backward launch failed"); }
+    std::swap(dcur, dnext);
   }
   if (loss) {
     if (cudaMemcpyAsync(loss, m->loss.p, sizeof(float), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
@@ -602,8 +773,8 @@ int twmc_mlp_adam(twmc_mlp* m, float lr, float beta1, float beta2, float eps, vo
   ++m->step;
   const float c1 = float(1.0 / (1.0 - std::pow(double(beta1), double(m->step))));
   const float c2 = float(1.0 / (1.0 - std::pow(double(beta2), double(m->step))));
-  adam_kernel<<<grid_for(m->nparam, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      m->w.p, m->w16.p, m->g.p, m->m.p, m->v.p, m->nparam, lr, beta1, beta2, eps, c1, c2);
+  adam_kernel<<<grid_for((m->nparam + 3) / 4, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+      m->w.p, m->w16.p, m->g.p, m->m.p, m->v.p, m->nparam, m->map, m->nl, lr, beta1, beta2, eps, c1, c2);
   ++m->launches;
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? TWMC_OK : mfail(m, TWMC_ERR_CUDA, cudaGetErrorString(e));
