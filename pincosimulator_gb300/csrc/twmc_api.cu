@@ -48,11 +48,11 @@ struct Matrix {
   std::vector<cd> base;   // n_sites
   std::vector<cd> amp;    // n_sites (noise amplitudes)
   int kind = TWMC_DISORDER_NONE;
-  bool uniform() const {
-    if (kind != TWMC_DISORDER_NONE) return false;
+  bool base_uniform() const {
     for (const cd& v : base) if (v != base[0]) return false;
     return true;
   }
+  bool uniform() const { return kind == TWMC_DISORDER_NONE && base_uniform(); }
 };
 
 struct DevBuf {
@@ -110,6 +110,7 @@ struct twmc_handle {
   cudaEvent_t fork = nullptr;
   cudaEvent_t snap_ready = nullptr, snap_free = nullptr;  // d_snap written (stream) / read (dl_stream)
   DevBuf d_snap;
+  DevBuf d_frames;         // all frames of a small run
   // page-locked host staging for fields copied row by row to the caller
   double* h_stage = nullptr;
   size_t h_stage_bytes = 0;
@@ -170,29 +171,27 @@ void read_matrix(const twmc_matrix& src, int64_t n, Matrix* m) {
 
 size_t rsize(int prec) { return prec ? sizeof(double) : sizeof(float); }
 
+// Uploads go on the handle's stream, in order with the kernels that read them
+// (copies from pageable memory return with the source staged).
+template <typename T>
+bool upload_raw(DevBuf* b, const T* data, size_t n, cudaStream_t s) {
+  if (!b->ensure(n * sizeof(T))) return false;
+  return cudaMemcpyAsync(b->p, data, n * sizeof(T), cudaMemcpyHostToDevice, s) == cudaSuccess;
+}
+
 // Upload complex values in the state precision.
-bool upload_c(DevBuf* b, const std::vector<cd>& v, int prec) {
+bool upload_c(DevBuf* b, const std::vector<cd>& v, int prec, cudaStream_t s) {
   const size_t n = v.size();
-  if (!b->ensure(n * 2 * rsize(prec))) return false;
-  if (prec) {
-    return cudaMemcpy(b->p, v.data(), n * sizeof(cd), cudaMemcpyHostToDevice) == cudaSuccess;
-  }
+  if (prec) return upload_raw(b, v.data(), n, s);
   std::vector<float> f(2 * n);
   for (size_t i = 0; i < n; ++i) { f[2 * i] = float(v[i].real()); f[2 * i + 1] = float(v[i].imag()); }
-  return cudaMemcpy(b->p, f.data(), f.size() * sizeof(float), cudaMemcpyHostToDevice) == cudaSuccess;
+  return upload_raw(b, f.data(), f.size(), s);
 }
 
-bool upload_r(DevBuf* b, const std::vector<double>& v, int prec) {
-  if (!b->ensure(v.size() * rsize(prec))) return false;
-  if (prec) return cudaMemcpy(b->p, v.data(), v.size() * sizeof(double), cudaMemcpyHostToDevice) == cudaSuccess;
+bool upload_r(DevBuf* b, const std::vector<double>& v, int prec, cudaStream_t s) {
+  if (prec) return upload_raw(b, v.data(), v.size(), s);
   std::vector<float> f(v.begin(), v.end());
-  return cudaMemcpy(b->p, f.data(), f.size() * sizeof(float), cudaMemcpyHostToDevice) == cudaSuccess;
-}
-
-template <typename T>
-bool upload_raw(DevBuf* b, const T* data, size_t n) {
-  if (!b->ensure(n * sizeof(T))) return false;
-  return cudaMemcpy(b->p, data, n * sizeof(T), cudaMemcpyHostToDevice) == cudaSuccess;
+  return upload_raw(b, f.data(), f.size(), s);
 }
 
 // NoisyMatrix::SetTemporalValue (NoisyMatrix.cpp:164-250).
@@ -303,7 +302,7 @@ int build_tables(twmc_handle* h) {
     std::vector<cd> tw;
     for (int64_t j = 0; j < M0; ++j) tw.push_back(std::polar(1.0, -2.0 * M_PI * double(j) / double(M0)));
     for (int64_t j = 0; j < M1; ++j) tw.push_back(std::polar(1.0, -2.0 * M_PI * double(j) / double(M1)));
-    if (!upload_c(&h->d_tw, tw, prec)) return fail(h, TWMC_ERR_NOMEM, "twiddle table upload");
+    if (!upload_c(&h->d_tw, tw, prec, h->stream)) return fail(h, TWMC_ERR_NOMEM, "twiddle table upload");
     // separable k-space table: [2J fy cos(2 pi ky / ny) / N for ky < M0 |
     // 2J fx cos(2 pi kx / nx) / N for kx < M1]; the kernel adds the two.
     // the FP32 kernel folds dt into the hopping term (local_update_fused)
@@ -312,7 +311,7 @@ int build_tables(twmc_handle* h) {
     std::vector<double> kt;
     for (int64_t k = 0; k < M0; ++k) kt.push_back(scale * fy * std::cos(2.0 * M_PI / double(h->ny) * double(k)));
     for (int64_t k = 0; k < M1; ++k) kt.push_back(scale * fx * std::cos(2.0 * M_PI / double(h->nx) * double(k)));
-    if (!upload_r(&h->d_ktab, kt, prec)) return fail(h, TWMC_ERR_NOMEM, "k table upload");
+    if (!upload_r(&h->d_ktab, kt, prec, h->stream)) return fail(h, TWMC_ERR_NOMEM, "k table upload");
     if (h->integrator == TWMC_INTEGRATOR_SPLIT) {
       // (exp(-i theta) - 1) / N, theta = 2J (fx cos(2 pi kx / nx) + fy cos(2 pi ky / ny)) dt, at every
       // position p of the forward plan's output (frequencies bit-reversed per dimension);
@@ -331,7 +330,7 @@ int build_tables(twmc_handle* h) {
         const double sh = std::sin(0.5 * th);
         kf[size_t(p)] = cd(-2.0 * sh * sh, -std::sin(th)) / double(h->nsites);
       }
-      if (!upload_c(&h->d_kfac, kf, prec)) return fail(h, TWMC_ERR_NOMEM, "split-step table upload");
+      if (!upload_c(&h->d_kfac, kf, prec, h->stream)) return fail(h, TWMC_ERR_NOMEM, "split-step table upload");
     }
   } else if (h->lattice == TWMC_LATTICE_LIEB) {
     // Coupling triplets of TWMCLiebSolver::Setup (TWMCLiebSolver.cpp:54-85).
@@ -371,15 +370,29 @@ int build_tables(twmc_handle* h) {
         else { idx[size_t(c * 4 + j)] = int(c); w[size_t(c * 4 + j)] = cd(0, 0); }
       }
     }
-    if (!upload_raw(&h->d_nbr_idx, idx.data(), idx.size())) return fail(h, TWMC_ERR_NOMEM, "neighbour upload");
-    if (!upload_c(&h->d_nbr_w, w, prec)) return fail(h, TWMC_ERR_NOMEM, "neighbour upload");
+    if (!upload_raw(&h->d_nbr_idx, idx.data(), idx.size(), h->stream)) return fail(h, TWMC_ERR_NOMEM, "neighbour upload");
+    if (!upload_c(&h->d_nbr_w, w, prec, h->stream)) return fail(h, TWMC_ERR_NOMEM, "neighbour upload");
   }
   if (h->timedep) {
     std::vector<cd> iv(h->ft_vals.size()), is(h->ft_slopes.size());
     for (size_t i = 0; i < iv.size(); ++i) iv[i] = cd(0, 1) * h->ft_vals[i];
     for (size_t i = 0; i < is.size(); ++i) is[i] = cd(0, 1) * h->ft_slopes[i];
-    if (!upload_c(&h->d_ft_vals, iv, prec) || !upload_c(&h->d_ft_slopes, is, prec))
+    if (!upload_c(&h->d_ft_vals, iv, prec, h->stream) || !upload_c(&h->d_ft_slopes, is, prec, h->stream))
       return fail(h, TWMC_ERR_NOMEM, "F(t) table upload");
+  }
+  // the matrices of the initial draws, the same for every batch of the handle
+  // (uniform ones go as scalars, see batch_init)
+  {
+    const Matrix* mats[3] = {&h->m_U, &h->m_omega, &h->m_F};
+    auto up = [&](DevBuf* b, const std::vector<cd>& v) {
+      return upload_raw(b, reinterpret_cast<const double*>(v.data()), 2 * v.size(), h->stream);
+    };
+    bool ok = (h->m_binit.base_uniform() || up(&h->d_binit, h->m_binit.base)) &&
+              (h->m_bsigma.base_uniform() || up(&h->d_bsigma, h->m_bsigma.base));
+    for (int m = 0; m < 3 && ok; ++m)
+      ok = (mats[m]->base_uniform() || up(&h->d_base[m], mats[m]->base)) &&
+           (mats[m]->kind == TWMC_DISORDER_NONE || up(&h->d_amp[m], mats[m]->amp));
+    if (!ok) return fail(h, TWMC_ERR_NOMEM, "matrix upload");
   }
   // shared (non-noisy, non-uniform) per-site parameters
   for (int k = 0; k < 3; ++k) {
@@ -395,7 +408,7 @@ int build_tables(twmc_handle* h) {
         v[size_t(p)] = cd(-x.imag(), x.real());
       }
     }
-    if (!upload_c(&h->d_shared_par[k], v, prec)) return fail(h, TWMC_ERR_NOMEM, "parameter upload");
+    if (!upload_c(&h->d_shared_par[k], v, prec, h->stream)) return fail(h, TWMC_ERR_NOMEM, "parameter upload");
   }
   return TWMC_OK;
 }
@@ -534,8 +547,9 @@ int reduce(twmc_handle* h) {
   return TWMC_OK;
 }
 
-// Allocates the batch and draws initial fields / disorder on the GPU.
-int batch_init(twmc_handle* h, const twmc_task_desc* tasks, size_t n) {
+// Allocates the batch and draws initial fields / disorder on the GPU. want_real:
+// which drawn realisations (U, omega, F) the caller will read.
+int batch_init(twmc_handle* h, const twmc_task_desc* tasks, size_t n, const bool (&want_real)[3]) {
   const int64_t N = h->nsites;
   const int prec = h->prec;
   h->ntraj = int64_t(n);
@@ -559,7 +573,7 @@ int batch_init(twmc_handle* h, const twmc_task_desc* tasks, size_t n) {
     ids[i] = uint32_t(tasks[i].id);
     if (tasks[i].ic_kind != ic) return fail(h, TWMC_ERR_INVALID, "tasks of one batch must share ic_kind");
   }
-  if (!upload_raw(&h->d_seeds, seeds.data(), n) || !upload_raw(&h->d_ids, ids.data(), n))
+  if (!upload_raw(&h->d_seeds, seeds.data(), n, h->stream) || !upload_raw(&h->d_ids, ids.data(), n, h->stream))
     return fail(h, TWMC_ERR_NOMEM, "seed upload");
   InitArgs ia;
   std::memset(&ia, 0, sizeof(ia));
@@ -573,19 +587,20 @@ int batch_init(twmc_handle* h, const twmc_task_desc* tasks, size_t n) {
   ia.lattice = h->lattice;
   ia.gamma = h->gamma;
   ia.detuning = h->detuning;
-  auto up_cd = [&](DevBuf* b, const std::vector<cd>& v) -> const double* {
-    if (!upload_raw(b, reinterpret_cast<const double*>(v.data()), 2 * v.size())) return nullptr;
-    return b->as<double>();
+  auto base_of = [](const Matrix& m, const DevBuf& b, double (&scalar)[2]) -> const double* {
+    scalar[0] = m.base.empty() ? 0.0 : m.base[0].real();
+    scalar[1] = m.base.empty() ? 0.0 : m.base[0].imag();
+    return b.as<double>();  // NULL: uniform
   };
-  ia.binit = up_cd(&h->d_binit, h->m_binit.base);
-  ia.bsigma = up_cd(&h->d_bsigma, h->m_bsigma.base);
+  ia.binit = base_of(h->m_binit, h->d_binit, ia.binit_s);
+  ia.bsigma = base_of(h->m_bsigma, h->d_bsigma, ia.bsigma_s);
   if (ic == TWMC_IC_GIVEN) {
     std::vector<double> g(size_t(2 * N) * n);
     for (size_t i = 0; i < n; ++i) {
       if (!tasks[i].init_field) return fail(h, TWMC_ERR_INVALID, "TWMC_IC_GIVEN task without init_field");
       std::memcpy(&g[size_t(2 * N) * i], tasks[i].init_field, sizeof(double) * size_t(2 * N));
     }
-    if (!upload_raw(&h->d_given, g.data(), g.size())) return fail(h, TWMC_ERR_NOMEM, "initial field upload");
+    if (!upload_raw(&h->d_given, g.data(), g.size(), h->stream)) return fail(h, TWMC_ERR_NOMEM, "initial field upload");
     ia.given = h->d_given.as<double>();
   }
   // Real part of rsl = Im(omega) - gamma/2 (Lieb: -Im(E) - gamma/2), and of
@@ -611,8 +626,8 @@ int batch_init(twmc_handle* h, const twmc_task_desc* tasks, size_t n) {
   const Matrix* mats[3] = {&h->m_U, &h->m_omega, &h->m_F};
   const uint32_t streams[3] = {kStreamU, kStreamOmega, kStreamF};
   for (int m = 0; m < 3; ++m) {
-    ia.base[m] = up_cd(&h->d_base[m], mats[m]->base);
-    ia.amp[m] = up_cd(&h->d_amp[m], mats[m]->amp);
+    ia.base[m] = base_of(*mats[m], h->d_base[m], ia.base_s[m]);
+    ia.amp[m] = h->d_amp[m].as<double>();
     ia.kind[m] = mats[m]->kind;
     ia.stream[m] = streams[m];
     const double* given_ptr[3] = {tasks[0].U_realization, tasks[0].omega_realization, tasks[0].F_realization};
@@ -623,7 +638,7 @@ int batch_init(twmc_handle* h, const twmc_task_desc* tasks, size_t n) {
         if (!src) return fail(h, TWMC_ERR_INVALID, "disorder realisations must be given for all tasks of a batch or none");
         std::memcpy(&g[size_t(2 * N) * i], src, sizeof(double) * size_t(2 * N));
       }
-      if (!upload_raw(&h->d_given_real[m], g.data(), g.size())) return fail(h, TWMC_ERR_NOMEM, "realisation upload");
+      if (!upload_raw(&h->d_given_real[m], g.data(), g.size(), h->stream)) return fail(h, TWMC_ERR_NOMEM, "realisation upload");
       ia.given_real[m] = h->d_given_real[m].as<double>();
     }
   }
@@ -640,6 +655,7 @@ int batch_init(twmc_handle* h, const twmc_task_desc* tasks, size_t n) {
     }
   }
   for (int m = 0; m < 3; ++m) {
+    if (!want_real[m]) continue;
     if (h->d_real_out[m].ensure(n * N * 2 * sizeof(double))) ia.real_out[m] = h->d_real_out[m].as<double>();
     else return fail(h, TWMC_ERR_NOMEM, "realisation allocation");
   }
@@ -671,6 +687,7 @@ int download_real(twmc_handle* h, const DevBuf& b, double* out, size_t n) {
 // strided copy.
 constexpr size_t kWideChunk = size_t(1) << 25;  // 256 MB of doubles
 constexpr int kFinalChunks = 4;                  // trajectory ranges of the final-field pipeline
+constexpr size_t kCollectMax = size_t(1) << 28;  // most bytes of frames collected on the device
 constexpr size_t kSnapMax = size_t(8) << 30;     // largest final field (bytes) the pipeline stages
 
 // m device rows of `row` doubles (consecutive) to host rows `row_stride`
@@ -720,21 +737,47 @@ int download_rows(twmc_handle* h, double* out, size_t row_stride) {
 // one host memcpy per trajectory. Frames of small runs and of any layout
 // take this route: a strided copy of short rows straight into pageable
 // memory cost about 1 ms per frame of 1000 x 64 sites.
+int ensure_stage(twmc_handle* h, size_t bytes) {
+  if (bytes <= h->h_stage_bytes) return TWMC_OK;
+  if (h->h_stage) cudaFreeHost(h->h_stage);
+  h->h_stage = nullptr;
+  h->h_stage_bytes = 0;
+  TWMC_CUDA(h, cudaHostAlloc(reinterpret_cast<void**>(&h->h_stage), bytes, cudaHostAllocDefault));
+  h->h_stage_bytes = bytes;
+  return TWMC_OK;
+}
+
 template <typename Dst>
 int download_scatter(twmc_handle* h, Dst dst) {
   const size_t rows = size_t(h->ntraj), row = size_t(2 * h->nsites);
   const size_t bytes = rows * row * sizeof(double);
-  if (bytes > h->h_stage_bytes) {
-    if (h->h_stage) cudaFreeHost(h->h_stage);
-    h->h_stage = nullptr;
-    h->h_stage_bytes = 0;
-    TWMC_CUDA(h, cudaHostAlloc(reinterpret_cast<void**>(&h->h_stage), bytes, cudaHostAllocDefault));
-    h->h_stage_bytes = bytes;
-  }
-  int rc = download_rows(h, h->h_stage, row);
+  int rc = ensure_stage(h, bytes);
+  if (rc) return rc;
+  rc = download_rows(h, h->h_stage, row);
   if (rc) return rc;
   TWMC_CUDA(h, cudaStreamSynchronize(h->stream));
   for (size_t r = 0; r < rows; ++r) std::memcpy(dst(r), h->h_stage + r * row, row * sizeof(double));
+  return TWMC_OK;
+}
+
+// The collected frames (rows of `row` doubles in d_frames) to the caller's rows:
+// straight into page-locked memory, else through the handle's page-locked
+// buffer.
+int download_collected(twmc_handle* h, double* out, size_t row_stride, size_t row, size_t rows) {
+  cudaPointerAttributes at;
+  const bool locked = cudaPointerGetAttributes(&at, out) == cudaSuccess && at.type == cudaMemoryTypeHost;
+  cudaGetLastError();
+  if (locked) {
+    TWMC_CUDA(h, copy_rows_d2h(h->device, out, row_stride, h->d_frames.p, row, rows, h->stream));
+    return TWMC_OK;
+  }
+  const size_t bytes = rows * row * sizeof(double);
+  int rc = ensure_stage(h, bytes);
+  if (rc) return rc;
+  TWMC_CUDA(h, cudaMemcpyAsync(h->h_stage, h->d_frames.p, bytes, cudaMemcpyDeviceToHost, h->stream));
+  TWMC_CUDA(h, cudaStreamSynchronize(h->stream));
+  if (row_stride == row) std::memcpy(out, h->h_stage, bytes);
+  else for (size_t r = 0; r < rows; ++r) std::memcpy(out + r * row_stride, h->h_stage + r * row, row * sizeof(double));
   return TWMC_OK;
 }
 
@@ -893,7 +936,7 @@ int twmc_batch_init(twmc_handle* h, const twmc_task_desc* tasks, size_t n) {
     cudaSetDevice(h->device);
     h->err.clear();
     h->noise_steps = 0;
-    return batch_init(h, tasks, n);
+    return batch_init(h, tasks, n, {false, false, false});
   } catch (const std::bad_alloc&) {
     return fail(h, TWMC_ERR_NOMEM, "host allocation failed");
   }
@@ -970,8 +1013,14 @@ int twmc_run(twmc_handle* h, const twmc_task_desc* tasks, size_t n, twmc_outputs
     const int64_t N = h->nsites;
     // group tasks by (t_start, t_end, store_initial, ic_kind)
     std::map<std::tuple<double, double, int, int>, std::vector<size_t>> groups;
-    for (size_t i = 0; i < n; ++i)
-      groups[{tasks[i].t_start, tasks[i].t_end, tasks[i].store_initial ? 1 : 0, tasks[i].ic_kind}].push_back(i);
+    std::vector<size_t>* at = nullptr;
+    for (size_t i = 0; i < n; ++i) {
+      const twmc_task_desc &t = tasks[i], &u = tasks[i ? i - 1 : 0];
+      // (neighbours mostly share their group: no lookup; NaN times never compare equal)
+      if (!at || !(t.t_start == u.t_start && t.t_end == u.t_end && !t.store_initial == !u.store_initial && t.ic_kind == u.ic_kind))
+        at = &groups[{t.t_start, t.t_end, t.store_initial ? 1 : 0, t.ic_kind}];
+      at->push_back(i);
+    }
     // frame stride of the output buffer: the largest n_frames of any group
     int64_t max_frames = 0;
     std::vector<Schedule> scheds;
@@ -992,7 +1041,9 @@ int twmc_run(twmc_handle* h, const twmc_task_desc* tasks, size_t n, twmc_outputs
       const size_t bn = idx.size();
       std::vector<twmc_task_desc> bt(bn);
       for (size_t i = 0; i < bn; ++i) bt[i] = tasks[idx[i]];
-      int rc = batch_init(h, bt.data(), bn);
+      double* real_dst[3] = {out ? out->U_realization : nullptr, out ? out->omega_realization : nullptr,
+                             out ? out->F_realization : nullptr};
+      int rc = batch_init(h, bt.data(), bn, {real_dst[0] != nullptr, real_dst[1] != nullptr, real_dst[2] != nullptr});
       if (rc) return rc;
       // deterministic noise for this group: [task][step][site]
       h->noise_steps = 0;
@@ -1003,7 +1054,7 @@ int twmc_run(twmc_handle* h, const twmc_task_desc* tasks, size_t n, twmc_outputs
           return fail(h, TWMC_ERR_INVALID, "noise buffer must hold n_tasks x steps x n_sites values (one task group)");
         std::vector<cd> nz(need);
         for (size_t i = 0; i < need; ++i) nz[i] = cd(h->noise_host[2 * i], h->noise_host[2 * i + 1]);
-        if (!upload_c(&h->d_noise, nz, h->prec)) return fail(h, TWMC_ERR_NOMEM, "noise upload");
+        if (!upload_c(&h->d_noise, nz, h->prec, h->stream)) return fail(h, TWMC_ERR_NOMEM, "noise upload");
         h->noise_steps = s.steps;
       }
       if (h->timedep) {
@@ -1017,14 +1068,12 @@ int twmc_run(twmc_handle* h, const twmc_task_desc* tasks, size_t n, twmc_outputs
           hint = seg.first;
         }
         std::vector<float> offs_f(offs.begin(), offs.end());
-        if (!upload_raw(&h->d_ft_id, ids.data(), ids.size()) || !upload_raw(&h->d_ft_dt, offs.data(), offs.size()) ||
-            !upload_raw(&h->d_ft_dt_f, offs_f.data(), offs_f.size()))
+        if (!upload_raw(&h->d_ft_id, ids.data(), ids.size(), h->stream) || !upload_raw(&h->d_ft_dt, offs.data(), offs.size(), h->stream) ||
+            !upload_raw(&h->d_ft_dt_f, offs_f.data(), offs_f.size(), h->stream))
           return fail(h, TWMC_ERR_NOMEM, "F(t) schedule upload");
       }
       // realisations of noisy matrices
-      TWMC_CUDA(h, cudaStreamSynchronize(h->stream));
-      double* real_dst[3] = {out ? out->U_realization : nullptr, out ? out->omega_realization : nullptr,
-                             out ? out->F_realization : nullptr};
+      if (real_dst[0] || real_dst[1] || real_dst[2]) TWMC_CUDA(h, cudaStreamSynchronize(h->stream));
       for (int m = 0; m < 3; ++m) {
         if (!real_dst[m]) continue;
         std::vector<double> tmp(size_t(bn * N * 2));
@@ -1044,6 +1093,14 @@ int twmc_run(twmc_handle* h, const twmc_task_desc* tasks, size_t n, twmc_outputs
       const bool stage = contiguous && h->prec == 0 && size_t(bn) * size_t(N) * 16 <= kSnapMax &&
                          int64_t(bn) * N >= (int64_t(1) << 20);
       bool dl_used = false;
+      // Frames of runs below that size, whose copies would cost more than the
+      // steps between them (1000 chains of 64 sites: 170 us of copy, wait and
+      // host scatter per frame against 137 us of steps): placed in the
+      // caller's [trajectory][frame][site] layout on the device and copied at
+      // the end in one piece.
+      const bool collect = !stage && contiguous && out && out->frames && s.n_frames > 0 && s.frames_written == s.n_frames &&
+                           size_t(bn) * size_t(s.n_frames) * size_t(N) * 16 <= kCollectMax &&
+                           h->d_frames.ensure(size_t(bn) * size_t(s.n_frames) * size_t(N) * 16);
       // copies into the caller's arrays may still be in flight when a group
       // ends early with an error: drain both streams on every exit
       struct Drain {
@@ -1153,9 +1210,10 @@ int twmc_run(twmc_handle* h, const twmc_task_desc* tasks, size_t n, twmc_outputs
           if (int64_t(bn) >= nb) {  // every block holds trajectories: one copy, no wait
             TWMC_CUDA(h, cudaMemcpyAsync(dst, h->d_moments.p, size_t(nb) * N * 3 * sizeof(double),
                                          cudaMemcpyDeviceToHost, h->stream));
-          } else {
-            r2 = twmc_batch_download(h, nullptr, dst);
-            if (r2) return r2;
+          } else {  // one block per trajectory, the others empty
+            TWMC_CUDA(h, cudaMemcpyAsync(dst, h->d_moments.p, bn * size_t(N) * 3 * sizeof(double), cudaMemcpyDeviceToHost,
+                                         h->stream));
+            std::memset(dst + bn * size_t(N) * 3, 0, (size_t(nb) - bn) * size_t(N) * 3 * sizeof(double));
           }
         }
         if (out && out->frames) {
@@ -1165,6 +1223,11 @@ int twmc_run(twmc_handle* h, const twmc_task_desc* tasks, size_t n, twmc_outputs
               if (r2) return r2;
             }
             frame_sent = false;
+          } else if (collect) {
+            std::string err;
+            if (!place_launch(h->prec, h->d_state.p, h->d_frames.as<double>() + size_t(f) * row, int64_t(bn), int64_t(row),
+                              int64_t(size_t(s.n_frames) * row), h->stream, &err))
+              return fail(h, TWMC_ERR_CUDA, err);
           } else {
             int r2 = download_scatter(h, [&](size_t i) { return out->frames + (idx[i] * max_frames + f) * N * 2; });
             if (r2) return r2;
@@ -1217,6 +1280,11 @@ int twmc_run(twmc_handle* h, const twmc_task_desc* tasks, size_t n, twmc_outputs
           rc = download_scatter(h, [&](size_t i) { return out->final_field + idx[i] * N * 2; });
           if (rc) return rc;
         }
+      }
+      if (collect) {
+        rc = download_collected(h, out->frames + idx[0] * size_t(max_frames) * row, size_t(max_frames) * row,
+                                size_t(s.n_frames) * row, bn);
+        if (rc) return rc;
       }
       std::vector<int> st(bn);
       TWMC_CUDA(h, cudaMemcpyAsync(st.data(), h->d_status.p, bn * sizeof(int), cudaMemcpyDeviceToHost, h->stream));

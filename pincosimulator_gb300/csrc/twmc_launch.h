@@ -74,6 +74,10 @@ bool init_launch(const InitArgs& a, cudaStream_t s, std::string* err);
 // out[k] = double(in[k]) for k < n (in: FP32 device array).
 bool widen_launch(const void* in, double* out, int64_t n, cudaStream_t s, std::string* err);
 
+// A frame of rows x row reals (state precision) into rows of doubles `stride` apart.
+bool place_launch(int prec, const void* in, double* out, int64_t rows, int64_t row, int64_t stride, cudaStream_t s,
+                  std::string* err);
+
 struct MomentArgs {
   int64_t ntraj, nsites;
   int prec;

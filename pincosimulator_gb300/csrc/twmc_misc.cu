@@ -152,6 +152,15 @@ __global__ void widen_kernel(const float* __restrict__ in, double* __restrict__ 
     out[k] = double(in[k]);
 }
 
+// One frame of a batch (n = trajectories x reals per trajectory values) into
+// its place among a trajectory's frames, as doubles: row r of the batch at
+// out + r * stride.
+template <typename R>
+__global__ void place_kernel(const R* __restrict__ in, double* __restrict__ out, int64_t n, int64_t row, int64_t stride) {
+  for (int64_t k = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; k < n; k += int64_t(gridDim.x) * blockDim.x)
+    out[(k / row) * stride + k % row] = double(in[k]);
+}
+
 }  // namespace
 
 bool init_launch(const InitArgs& a, cudaStream_t s, std::string* err) {
@@ -220,6 +229,16 @@ bool widen_launch(const void* in, double* out, int64_t n, cudaStream_t s, std::s
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) { if (err) *err = std::string("widen: ") + cudaGetErrorString(e); return false; }
   return true;
+}
+
+bool place_launch(int prec, const void* in, double* out, int64_t rows, int64_t row, int64_t stride, cudaStream_t s,
+                  std::string* err) {
+  const int64_t n = rows * row;
+  if (n <= 0) return true;
+  const int grid = int(std::min<int64_t>((n + 255) / 256, 152 * 16));
+  if (prec == 0) place_kernel<float><<<grid, 256, 0, s>>>(static_cast<const float*>(in), out, n, row, stride);
+  else place_kernel<double><<<grid, 256, 0, s>>>(static_cast<const double*>(in), out, n, row, stride);
+  return check(cudaGetLastError(), err, "place_kernel");
 }
 
 }  // namespace twmc
