@@ -12,18 +12,14 @@
 
 namespace twmc {
 
-// Threads per CTA: whole trajectories, up to 256 threads, with the two
-// exchange buffers and the state slices of all trajectories of the CTA inside
-// a ~100 KB shared-memory budget.
+// Threads per CTA: one trajectory, or as many short ones as fill a warp. No
+// more: a barrier then waits for one trajectory's warps only, and an SM fills
+// up to its last free registers and a batch to its last SM (16x16 with 2500
+// trajectories in 128-thread CTAs: 313 of them on 304 places, two rounds).
 template <typename R, class P>
 constexpr int cta_for() {
   constexpr int tpt = PlanInfo<P>::TPT;
-  constexpr size_t per_traj = (sizeof(R) == 4 ? 3 : 2) * sizeof(c2_t<R>) * size_t(PlanInfo<P>::N) * 17 / 16;
-  // FP64: the FP64 pipe of an SM is one for all its warps, so one warp (or one
-  // trajectory) per CTA balances the SMs best
-  int tpc = sizeof(R) == 8 ? (tpt >= 32 ? 1 : 32 / tpt) : tpt >= 256 ? 1 : 256 / tpt;
-  while (tpc > 1 && size_t(tpc) * per_traj > 100 * 1024) tpc /= 2;
-  return tpc * tpt;
+  return tpt >= 32 ? tpt : 32;
 }
 
 template <typename R, class P, bool FAST, bool SPLIT = false>

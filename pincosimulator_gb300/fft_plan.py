@@ -250,12 +250,22 @@ def fp64_bits(n: int) -> int:
     return 2 if n <= 8 else 3 if n <= 10 else 4
 
 
+def fp32_bits(n: int) -> int:
+    """Register bits of the FP32 plan of 2^n sites: 16 sites per thread (fewest
+    exchanges), but 8 up to 128 sites, where that costs nothing on a full device
+    and halves a step's latency on a part-filled one. GB300, us per step with 16
+    and 8 sites per thread: 1x32 with 100 trajectories 1.16 / 0.53, with 20000
+    3.30 / 2.07; 1x64 with 1000 1.23 / 0.63, with 16000 4.04 / 4.13; 1x128 with 300
+    1.23 / 0.66, with 8000 3.99 / 3.71; but 1x256 with 6000 5.98 / 11.2."""
+    return 3 if n <= 7 else 4
+
+
 def emit_header() -> str:
     """C++ source with the constexpr plans of every supported shape:
     Plan_<bx>_<by> (FP32) and PlanD_<bx>_<by> (FP64)."""
     lines = ["// Generated by pincosimulator_gb300/fft_plan.py -- do not edit.", "#pragma once", "namespace twmc {"]
     for (bx, by) in SUPPORTED_SHAPES:
-        lines += _emit_plan(f"Plan_{bx}_{by}", make_plan(bx, by, 4))
+        lines += _emit_plan(f"Plan_{bx}_{by}", make_plan(bx, by, fp32_bits(bx + by)))
     for (bx, by) in SUPPORTED_SHAPES:
         lines += _emit_plan(f"PlanD_{bx}_{by}", make_plan(bx, by, fp64_bits(bx + by)))
     lines.append("}  // namespace twmc")
