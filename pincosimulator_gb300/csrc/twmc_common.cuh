@@ -160,6 +160,31 @@ __device__ __forceinline__ float2 normal_pair(uint32_t a, uint32_t b, float) {
   return scaled_normal_pair(a, b, kNegTwoLn2);
 }
 
+// float -> double and back (round to nearest even) by integer operations, the
+// conversion instructions for subnormals, infinities and NaN only: those run
+// on the FP64 pipe, two lanes per SM and cycle on GB300 (in functions of their
+// own: the compiler would predicate them, and predicated instructions still
+// take their turn on that pipe).
+static __device__ __noinline__ double widen_rare(float x) { return double(x); }
+static __device__ __noinline__ float narrow_rare(double x) { return float(x); }
+static __device__ __noinline__ double fma_rare(double a, double b, double c) { return fma(a, b, c); }
+__device__ __forceinline__ double widen(float x) {
+  const uint32_t b = __float_as_uint(x), e = b & 0x7f800000u;
+  if (e == 0u || e == 0x7f800000u) return widen_rare(x);
+  return __hiloint2double(int((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + 0x38000000u)), int(b << 29));
+}
+__device__ __forceinline__ float narrow(double x) {
+  const uint32_t hi = uint32_t(__double2hiint(x)), lo = uint32_t(__double2loint(x));
+  const uint32_t e = (hi >> 20) & 0x7ffu;
+  if (e - 897u > 252u) return narrow_rare(x);  // outside 2^-126 <= |x| < 2^127
+  const uint32_t m = ((e - 896u) << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29), rest = lo & 0x1fffffffu;
+  const uint32_t up = rest > 0x10000000u || (rest == 0x10000000u && (m & 1u)) ? 1u : 0u;
+  return __uint_as_float((hi & 0x80000000u) | (m + up));
+}
+
+// Whether x is +0 or -0, without a comparison on the FP64 pipe.
+__device__ __forceinline__ bool is_zero(double x) { return ((__double2hiint(x) & 0x7fffffff) | __double2loint(x)) == 0; }
+
 // Box-Muller, FP64: u = (w + 1/2) 2^-32.
 __device__ __forceinline__ double2 normal_pair(uint32_t a, uint32_t b, double) {
   const double u1 = (double(a) + 0.5) * 0x1p-32;

@@ -286,14 +286,6 @@ __global__ void hbatch_moments_kernel(const MomentArgs* __restrict__ ma) {
   moments_site<float>(a, p, int(blockIdx.y));
 }
 
-// FP64 of a float by integer operations (subnormals, infinities and NaN by the
-// conversion): conversions run on the FP64 pipe, which bounds the sums below.
-__device__ __forceinline__ double widen(float x) {
-  const uint32_t b = __float_as_uint(x), e = b & 0x7f800000u;
-  if (e == 0u || e == 0x7f800000u) return double(x);
-  return __hiloint2double(int((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + 0x38000000u)), int(b << 29));
-}
-
 // Compensated FP64 sum as KSum (Neumaier), the larger operand chosen by the
 // integer order of the magnitudes' upper words: equal upper words mean equal
 // exponents, where either order recovers the rounding error exactly.

@@ -18,76 +18,91 @@ __device__ __forceinline__ double2 ld_c(const double* p, int64_t i) { return mak
 // FP64 runs with the FP64 one; the sums with the base values are FP64 in
 // both. (The FP64 logarithm and sine / cosine of two draws per site took
 // 20 ms for 16384 trajectories of 64 x 64 on GB300's narrow FP64 pipe.)
-__device__ __forceinline__ double2 init_normal(uint32_t a, uint32_t b, int prec) {
-  if (prec == 0) {
+template <int PREC>
+__device__ __forceinline__ double2 init_normal(uint32_t a, uint32_t b) {
+  if constexpr (PREC == 0) {
     const float2 z = normal_pair(a, b, 0.0f);
-    return make_double2(double(z.x), double(z.y));
+    return make_double2(widen(z.x), widen(z.y));
+  } else {
+    return normal_pair(a, b, 0.0);
   }
-  return normal_pair(a, b, 0.0);
 }
+// One thread per pair of sites (p, p + half), which share each stream's Philox
+// call. The FP64 pipe bounds it on FP32 runs too: what is zero (imaginary parts
+// of spread and amplitude) or not asked for (matrices without disorder, array
+// or realisation) is left out, and conversions are integer operations; 16384
+// trajectories of 64 x 64 with omega disorder took 2.6 ms with one thread per
+// site and all three matrices formed.
+template <int PREC>
+__device__ __forceinline__ void store_c(void* p, int64_t i, double2 v) {
+  if constexpr (PREC == 0) reinterpret_cast<float2*>(p)[i] = make_float2(narrow(v.x), narrow(v.y));
+  else reinterpret_cast<double2*>(p)[i] = v;
+}
+template <int PREC>
 __global__ void init_kernel(const InitArgs a) {
-  const int64_t total = a.ntraj * a.nsites;
-  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < total; i += int64_t(gridDim.x) * blockDim.x) {
-    const int64_t tr = i / a.nsites, p = i % a.nsites;
+  const int64_t half = (a.nsites + 1) / 2, total = a.ntraj * half;
+  const double half_gamma = a.gamma / 2.0;
+  for (int64_t k = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; k < total; k += int64_t(gridDim.x) * blockDim.x) {
+    const int64_t tr = total <= 0xffffffffll ? int64_t(uint32_t(k) / uint32_t(half)) : k / half, c0 = k - tr * half;
     const uint32_t seed = a.seeds[tr], id = a.ids[tr];
-    int hi;
-    const uint32_t c0 = site_ctr(p, a.nsites, &hi);
-    double2 b;
-    if (a.ic_kind == 2) {
-      b = ld_c(a.given, i);
-    } else {
-      b = a.binit ? ld_c(a.binit, p) : make_double2(a.binit_s[0], a.binit_s[1]);
-      if (a.ic_kind == 0) {
-        const u32x4 w = philox4x32_10(u32x4{c0, 0u, kStreamInit, 0u}, seed, id);
-        const double2 z = hi ? init_normal(w.z, w.w, a.prec) : init_normal(w.x, w.y, a.prec);
-        const double2 sg = a.bsigma ? ld_c(a.bsigma, p) : make_double2(a.bsigma_s[0], a.bsigma_s[1]);
-        b = cadd(b, cmul(sg, z));
-      }
-    }
-    double2 v[3];
-#pragma unroll
-    for (int m = 0; m < 3; ++m) {
-      if (a.given_real[m]) {
-        v[m] = ld_c(a.given_real[m], i);
-        continue;
-      }
-      v[m] = a.base[m] ? ld_c(a.base[m], p) : make_double2(a.base_s[m][0], a.base_s[m][1]);
-      if (a.kind[m] != 0) {
-        const u32x4 w = philox4x32_10(u32x4{c0, 0u, a.stream[m], 0u}, seed, id);
-        const double2 amp = ld_c(a.amp[m], p);
-        if (a.kind[m] == 1) {
-          const double2 z = hi ? init_normal(w.z, w.w, a.prec) : init_normal(w.x, w.y, a.prec);
-          v[m].x += z.x * amp.x;
-          v[m].y += z.y * amp.y;
-        } else {
-          const uint32_t u0 = hi ? w.z : w.x, u1 = hi ? w.w : w.y;
-          v[m].x += double(u0) * 0x1p-32 * amp.x;
-          v[m].y += double(u1) * 0x1p-32 * amp.y;
+    const int ns = c0 + half < a.nsites ? 2 : 1;
+    u32x4 w{};
+    if (a.ic_kind == 0) w = philox4x32_10(u32x4{uint32_t(c0), 0u, kStreamInit, 0u}, seed, id);
+    for (int s = 0; s < ns; ++s) {
+      const int64_t p = c0 + s * half, i = tr * a.nsites + p;
+      double2 b;
+      if (a.ic_kind == 2) {
+        b = ld_c(a.given, i);
+      } else {
+        b = a.binit ? ld_c(a.binit, p) : make_double2(a.binit_s[0], a.binit_s[1]);
+        if (a.ic_kind == 0) {
+          const double2 z = s ? init_normal<PREC>(w.z, w.w) : init_normal<PREC>(w.x, w.y);
+          const double2 sg = a.bsigma ? ld_c(a.bsigma, p) : make_double2(a.bsigma_s[0], a.bsigma_s[1]);
+          double2 e = make_double2(__dmul_rn(sg.x, z.x), __dmul_rn(sg.x, z.y));
+          if (!is_zero(sg.y)) e = make_double2(fma_rare(-sg.y, z.y, e.x), fma_rare(sg.y, z.x, e.y));
+          b = cadd(b, e);
         }
       }
+      store_c<PREC>(a.state, i, b);
     }
 #pragma unroll
-    for (int m = 0; m < 3; ++m)
-      if (a.real_out[m]) { a.real_out[m][2 * i] = v[m].x; a.real_out[m][2 * i + 1] = v[m].y; }
-    // v[0] = U, v[1] = omega (Lieb: E), v[2] = F
-    double2 rsl;
-    if (a.lattice == 0) rsl = make_double2(v[1].y - a.gamma / 2.0, -v[1].x);     // -i omega - gamma/2
-    else {
-      const double2 d = make_double2(a.detuning - v[1].x, -v[1].y);            // detuning - E
-      rsl = make_double2(d.y - a.gamma / 2.0, -d.x);                            // -i delta - gamma/2
-    }
-    const double2 iU = make_double2(-v[0].y, v[0].x);
-    const double2 iF = make_double2(-v[2].y, v[2].x);
-    if (a.prec == 0) {
-      reinterpret_cast<float2*>(a.state)[i] = make_float2(float(b.x), float(b.y));
-      if (a.rsl) reinterpret_cast<float2*>(a.rsl)[i] = make_float2(float(rsl.x), float(rsl.y));
-      if (a.iU) reinterpret_cast<float2*>(a.iU)[i] = make_float2(float(iU.x), float(iU.y));
-      if (a.iF) reinterpret_cast<float2*>(a.iF)[i] = make_float2(float(iF.x), float(iF.y));
-    } else {
-      reinterpret_cast<double2*>(a.state)[i] = b;
-      if (a.rsl) reinterpret_cast<double2*>(a.rsl)[i] = rsl;
-      if (a.iU) reinterpret_cast<double2*>(a.iU)[i] = iU;
-      if (a.iF) reinterpret_cast<double2*>(a.iF)[i] = iF;
+    for (int m = 0; m < 3; ++m) {  // U, omega (Lieb: E), F
+      void* const dst = m == 0 ? a.iU : m == 1 ? a.rsl : a.iF;
+      if (!dst && !a.real_out[m]) continue;
+      const bool draw = !a.given_real[m] && a.kind[m] != 0;
+      u32x4 u{};
+      if (draw) u = philox4x32_10(u32x4{uint32_t(c0), 0u, a.stream[m], 0u}, seed, id);
+      for (int s = 0; s < ns; ++s) {
+        const int64_t p = c0 + s * half, i = tr * a.nsites + p;
+        double2 v;
+        if (a.given_real[m]) {
+          v = ld_c(a.given_real[m], i);
+        } else {
+          v = a.base[m] ? ld_c(a.base[m], p) : make_double2(a.base_s[m][0], a.base_s[m][1]);
+          if (draw) {
+            uint32_t u0 = s ? u.z : u.x, u1 = s ? u.w : u.y;
+            const double2 amp = ld_c(a.amp[m], p);
+            if (a.kind[m] == 1) {
+              const double2 z = init_normal<PREC>(u0, u1);
+              v.x += z.x * amp.x;
+              if (!is_zero(amp.y)) v.y = fma_rare(z.y, amp.y, v.y);
+            } else {
+              asm volatile("" : "+r"(u0), "+r"(u1));  // (stays in this branch)
+              v.x += double(u0) * 0x1p-32 * amp.x;
+              if (!is_zero(amp.y)) v.y = fma_rare(double(u1) * 0x1p-32, amp.y, v.y);
+            }
+          }
+        }
+        if (a.real_out[m]) { a.real_out[m][2 * i] = v.x; a.real_out[m][2 * i + 1] = v.y; }
+        if (!dst) continue;
+        if (m == 1) {  // rsl
+          if (a.lattice == 0) v = make_double2(v.y - half_gamma, -v.x);  // -i omega - gamma/2
+          else v = make_double2(-v.y - half_gamma, -(a.detuning - v.x));  // -i (detuning - E) - gamma/2
+        } else {       // i U, i F
+          v = make_double2(-v.y, v.x);
+        }
+        store_c<PREC>(dst, i, v);
+      }
     }
   }
 }
@@ -164,10 +179,11 @@ __global__ void place_kernel(const R* __restrict__ in, double* __restrict__ out,
 }  // namespace
 
 bool init_launch(const InitArgs& a, cudaStream_t s, std::string* err) {
-  const int64_t total = a.ntraj * a.nsites;
+  const int64_t total = a.ntraj * ((a.nsites + 1) / 2);
   if (total <= 0) return true;
   const int64_t blocks = std::min<int64_t>((total + 255) / 256, 152 * 32);
-  init_kernel<<<int(blocks), 256, 0, s>>>(a);
+  if (a.prec == 0) init_kernel<0><<<int(blocks), 256, 0, s>>>(a);
+  else init_kernel<1><<<int(blocks), 256, 0, s>>>(a);
   return check(cudaGetLastError(), err, "init_kernel");
 }
 
