@@ -1,6 +1,7 @@
 """Builds libtwmc_cuda.so (the C-ABI CUDA library) in-tree for sm_103a.
 
-Steps: emit csrc/fft_plans.inc from fft_plan.py, compile every csrc/*.cu
+Steps: emit csrc/fft_plans.inc from fft_plan.py and csrc/bm_tables.inc from
+bm_tables.py, compile every csrc/*.cu
 with nvcc (one -gencode, translation units in parallel), link a shared
 library into pincosimulator_gb300/_build/. No cmake; runs the same on the
 x86 build container and the Arm GPU host.
@@ -29,13 +30,13 @@ SOURCES = ["twmc_api.cu", "twmc_square_f32.cu", "twmc_square_f64.cu", "twmc_ell.
 
 def _write_plans() -> None:
     sys.path.insert(0, os.path.dirname(HERE))
-    from pincosimulator_gb300 import fft_plan
+    from pincosimulator_gb300 import bm_tables, fft_plan
 
-    text = fft_plan.emit_header()
-    dst = os.path.join(CSRC, "fft_plans.inc")
-    if not os.path.exists(dst) or open(dst).read() != text:
-        with open(dst, "w") as f:
-            f.write(text)
+    for name, text in (("fft_plans.inc", fft_plan.emit_header()), ("bm_tables.inc", bm_tables.emit_header())):
+        dst = os.path.join(CSRC, name)
+        if not os.path.exists(dst) or open(dst).read() != text:
+            with open(dst, "w") as f:
+                f.write(text)
 
 
 def _deps_hash() -> str:
