@@ -157,6 +157,25 @@ __device__ __forceinline__ bool hb_next(const StepArgs* __restrict__ pts, const 
   return true;
 }
 
+// The packed body as a function of its own: inlined into a queue's item loop,
+// its step loop copied the operands of most packed instructions (60
+// instructions per site-update at every split, a third of them register
+// moves); as a function it is the single system's loop (43 to 48). A CTA that
+// holds whole trajectories copies the arguments to registers first; the
+// cluster splits, with 8 sites per thread more, read them from shared memory.
+// Site-updates/s inlined, by reference, by value: 64x64 4.06, 4.72, 4.67e11;
+// 32x32 3.87, 4.39, 4.76e11; 1x1024 4.85, 5.05e11 (the last two); 16x16 3.46,
+// 3.80e11; 1x32 3.02, 3.10e11; 128x128 3.53, 3.93, 3.70e11.
+template <int V, int NB, bool CH, int CL = 1>
+__device__ __noinline__ void hb_pair(const StepArgs& a, unsigned char* smem_raw, int64_t group) {
+  if constexpr (CL == 1) {
+    const StepArgs b = a;
+    pair_body<V, NB, CH, PAIR_SCALAR>(b, smem_raw, group);
+  } else {
+    pair_body<V, NB, CH, PAIR_SCALAR, CL>(a, smem_raw, group);
+  }
+}
+
 // 256-thread queue: register-FFT plans and real-space stencils.
 __global__ void __launch_bounds__(HB_CTA, 2)
 hbatch_kernel(const StepArgs* __restrict__ pts, const int* __restrict__ pvar, const int* __restrict__ pshape,
@@ -181,7 +200,7 @@ hbatch_kernel(const StepArgs* __restrict__ pts, const int* __restrict__ pvar, co
       default:
         switch (pshape[w.x]) {
 #define TWMC_HB_CASE(V, NB, CH) \
-  case TWMC_HB_CODE(V, NB, CH, 1): pair_body<V, NB, CH, PAIR_SCALAR>(s_a, smem_raw, w.y); break;
+  case TWMC_HB_CODE(V, NB, CH, 1): hb_pair<V, NB, CH>(s_a, smem_raw, w.y); break;
           TWMC_HB_SPLITS_256(TWMC_HB_CASE)
 #undef TWMC_HB_CASE
           default:
@@ -208,7 +227,7 @@ hbatch_kernel_512(const StepArgs* __restrict__ pts, const int* __restrict__ psha
   while (hb_next(pts, items, nitems, counter, s_a, s_item, cur, w, reload)) {
     switch (pshape[w.x]) {
 #define TWMC_HB_CASE(V, NB, CH) \
-  case TWMC_HB_CODE(V, NB, CH, 1): pair_body<V, NB, CH, PAIR_SCALAR>(s_a, smem_raw, w.y); break;
+  case TWMC_HB_CODE(V, NB, CH, 1): hb_pair<V, NB, CH>(s_a, smem_raw, w.y); break;
       TWMC_HB_SPLITS_512(TWMC_HB_CASE)
 #undef TWMC_HB_CASE
       default: ell_body<float, 8, 512, 1, true>(s_a, smem_raw, w.y, kOneGroup); break;
@@ -254,10 +273,10 @@ hbatch_cluster_kernel(const StepArgs* __restrict__ pts, const int* __restrict__ 
   __shared__ int s_item;
   hb_cluster_loop<2>(pts, items, nitems, counter, s_a, s_item, [&](int2 w) {
     switch (pshape[w.x]) {
-      case TWMC_HB_CODE(4, 1, false, 2): pair_body<4, 1, false, PAIR_SCALAR, 2>(s_a, smem_raw, w.y); break;
-      case TWMC_HB_CODE(5, 1, false, 2): pair_body<5, 1, false, PAIR_SCALAR, 2>(s_a, smem_raw, w.y); break;
-      case TWMC_HB_CODE(3, 1, false, 2): pair_body<3, 1, false, PAIR_SCALAR, 2>(s_a, smem_raw, w.y); break;
-      case TWMC_HB_CODE(1, 1, false, 2): pair_body<1, 1, false, PAIR_SCALAR, 2>(s_a, smem_raw, w.y); break;
+      case TWMC_HB_CODE(4, 1, false, 2): hb_pair<4, 1, false, 2>(s_a, smem_raw, w.y); break;
+      case TWMC_HB_CODE(5, 1, false, 2): hb_pair<5, 1, false, 2>(s_a, smem_raw, w.y); break;
+      case TWMC_HB_CODE(3, 1, false, 2): hb_pair<3, 1, false, 2>(s_a, smem_raw, w.y); break;
+      case TWMC_HB_CODE(1, 1, false, 2): hb_pair<1, 1, false, 2>(s_a, smem_raw, w.y); break;
       default:
         if (pvar[w.x] == kVarClusterPow2) ell_cluster_pow2_body<1024, true>(s_a, smem_raw, w.y, kOneGroup);
         else ell_cluster_body<float, 1024>(s_a, smem_raw, w.y, kOneGroup);
@@ -275,7 +294,7 @@ hbatch_cluster4_kernel(const StepArgs* __restrict__ pts, const int2* __restrict_
   __shared__ __align__(16) StepArgs s_a;
   __shared__ int s_item;
   hb_cluster_loop<4>(pts, items, nitems, counter, s_a, s_item,
-                     [&](int2 w) { pair_body<8, 1, false, PAIR_SCALAR, 4>(s_a, smem_raw, w.y); });
+                     [&](int2 w) { hb_pair<8, 1, false, 4>(s_a, smem_raw, w.y); });
 }
 
 // FP64 moment blocks of every point: grid (site chunk, block, point).
