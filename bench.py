@@ -201,7 +201,7 @@ def measure_other_paths(twmc, torch, sm_mhz=None):
     workload on the real-space stencil kernel (the same hopping operator
     applied without the FFT), the 256-point heterogeneous batch to t = 60,
     the 1-D Lieb lattice (256 cells, U disorder, F(t) ramp, 8192
-    trajectories) and the 128 x 128 lattice on the 2-CTA cluster kernel
+    trajectories) and the 128 x 128 lattice on the cluster kernel
     (4096 trajectories), each with its issue-rate fraction; the Lieb workload
     also through twmc_run (host wall clock, initial draws included)."""
     from pincosimulator_gb300 import workloads
@@ -210,8 +210,7 @@ def measure_other_paths(twmc, torch, sm_mhz=None):
     s = workloads.time_batch(sysd, NTRAJ, 2)
     r = FRAME_STEPS * NTRAJ * NX * NY * 2 / s
     out["headline_real_space"] = {"value": r, "unit": METRIC, "kernel": sysd.kernel_name, "ms_per_frame": s * 500}
-    prof = "rowrun_kernel_64x64.md" if sysd.kernel_name == "rowrun_kernel" else "ell_kernel_64x64_stencil.md"
-    out["headline_real_space"]["issue"] = issue_fraction(r, prof, sm_mhz, torch)
+    out["headline_real_space"]["issue"] = issue_fraction(r, "pair_kernel_64x64.md", sm_mhz, torch)
     sysd.close()
     out["heterogeneous_batch"] = measure_batch(twmc, torch, sm_mhz)
     sysd = workloads.lieb()
@@ -226,7 +225,7 @@ def measure_other_paths(twmc, torch, sm_mhz=None):
     out["lieb"] = {"value": r, "unit": METRIC, "kernel": sysd.kernel_name, "kernel_ms_per_1000_steps": kms,
                    "workload": "1-D Lieb 256 cells x 3, PBC, U = 0.27 + 0.06 U[0,1), F(t) ramp on B sites, "
                                "8192 trajectories, 1000 steps (CUDA events around the step launches)",
-                   "issue": issue_fraction(r, "lieb_cell_kernel_lieb768.md", sm_mhz, torch),
+                   "issue": issue_fraction(r, "lieb_pair_kernel_lieb768.md", sm_mhz, torch),
                    "twmc_run": {"value": sysd.n_sites * 8192 * 1000 / el, "unit": METRIC,
                                 "timing": "host wall clock around the twmc_run call (initial draws and frame "
                                           "bookkeeping included)"}}
@@ -236,7 +235,7 @@ def measure_other_paths(twmc, torch, sm_mhz=None):
     r = 128 * 128 * 4096 * FRAME_STEPS / s
     out["square128"] = {"value": r, "unit": METRIC, "kernel": sysd.kernel_name, "ms_per_frame": s * 1e3,
                         "workload": "128x128 PBC, the headline parameters, 4096 trajectories, one 250-step frame",
-                        "issue": issue_fraction(r, "ell_cluster_pow2_kernel_128x128.md", sm_mhz, torch)}
+                        "issue": issue_fraction(r, "pair_cluster_kernel_128x128.md", sm_mhz, torch)}
     sysd.close()
     return out
 

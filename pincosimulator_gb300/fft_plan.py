@@ -246,7 +246,8 @@ def fp64_bits(n: int) -> int:
     16x16 with 500 trajectories 3.25 / 3.12 / 1.82, 1x64 with 200 0.74 / 0.37 /
     0.19, 1x512 with 600 2.80 / 3.60 / 3.36 (more twiddles are thread-dependent
     products on 4 sites), 32x32 with 700 3.15 / 3.35 / 2.82, 64x64 with 300
-    3.24 / 3.24 / 3.29."""
+    3.24 / 3.24 / 3.29 (all with library log and sincos in the draws; with the
+    tabulated draws the choices run 16x16 at 4.52, 1x512 at 4.86, 64x64 at 4.31)."""
     return 2 if n <= 8 else 3 if n <= 10 else 4
 
 

@@ -3,8 +3,8 @@
 * ``square64``  -- 2-D 64x64 PBC, J=1, U=0.2, gamma=1, omega=-0.5 with
   Gaussian disorder of amplitude 0.2, F=2, dt=0.002, frames of 250 steps
   (the headline workload; ``--hop stencil`` for the real-space kernel).
-* ``square128`` -- the same parameters on a 128x128 lattice (the 2-CTA
-  cluster stencil kernel, power-of-two form).
+* ``square128`` -- the same parameters on a 128x128 lattice (the cluster
+  stencil kernel).
 * ``chain64``   -- the 1-D chain of 64 sites, J=1, U=0.1, gamma=1, omega=-1,
   F=1.5, beta_init_sigma=0.5, dt=0.005, a frame every 100 steps: the
   configuration of the reference's own CPU runs (1000 trajectories to
