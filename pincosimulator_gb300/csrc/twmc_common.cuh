@@ -100,9 +100,10 @@ __device__ __forceinline__ void static_for(F&& f) {
 // ---------------------------------------------------------------------------
 struct u32x4 { uint32_t x, y, z, w; };
 
-__host__ __device__ __forceinline__ u32x4 philox4x32_10(u32x4 c, uint32_t k0, uint32_t k1) {
+template <int ROUNDS>
+__host__ __device__ __forceinline__ u32x4 philox4x32(u32x4 c, uint32_t k0, uint32_t k1) {
 #pragma unroll
-  for (int r = 0; r < 10; ++r) {
+  for (int r = 0; r < ROUNDS; ++r) {
 #ifdef __CUDA_ARCH__
     const uint32_t lo0 = 0xD2511F53u * c.x, hi0 = __umulhi(0xD2511F53u, c.x);
     const uint32_t lo1 = 0xCD9E8D57u * c.z, hi1 = __umulhi(0xCD9E8D57u, c.z);
@@ -118,6 +119,10 @@ __host__ __device__ __forceinline__ u32x4 philox4x32_10(u32x4 c, uint32_t k0, ui
   return c;
 }
 
+__host__ __device__ __forceinline__ u32x4 philox4x32_10(u32x4 c, uint32_t k0, uint32_t k1) {
+  return philox4x32<10>(c, k0, k1);
+}
+
 // Noise streams (counter word 2).
 enum : uint32_t { kStreamWiener = 0, kStreamInit = 1, kStreamU = 2, kStreamOmega = 3, kStreamF = 4 };
 
@@ -131,6 +136,31 @@ constexpr uint32_t kWienerKey0 = 0x243F6A88u, kWienerKey1 = 0x85A308D3u;
 
 __host__ __device__ __forceinline__ u32x4 wiener_words(uint32_t pair, uint32_t step, uint32_t seed, uint32_t id) {
   return philox4x32_10(u32x4{pair, step, id, seed}, kWienerKey0, kWienerKey1);
+}
+
+// The Wiener words of one site pair over many steps. Of the ten rounds' twenty
+// 32 x 32 -> 64-bit products (four cycles each on the FMA pipe's wide half,
+// two thirds of the packed steps' time there) the first three rounds hold four
+// that do not depend on the step and one that all pairs of a trajectory share: a
+// thread keeps what they give per pair (WienerSite, four registers) and forms
+// the shared one once per step (WienerStep). The same words as wiener_words.
+struct WienerSite { uint32_t a, b, c, d; };
+struct WienerStep { uint32_t hi, lo; };
+constexpr uint32_t kPhiloxM0 = 0xD2511F53u, kPhiloxM1 = 0xCD9E8D57u, kPhiloxW0 = 0x9E3779B9u, kPhiloxW1 = 0xBB67AE85u;
+__device__ __forceinline__ WienerSite wiener_site(uint32_t pair, uint32_t seed, uint32_t id) {
+  const uint32_t y = __umulhi(kPhiloxM0, pair) ^ seed ^ kWienerKey1;
+  const uint32_t s0 = __umulhi(kPhiloxM1, y) ^ (kPhiloxM1 * id) ^ (kWienerKey0 + kPhiloxW0);
+  return WienerSite{(kPhiloxM0 * pair) ^ (kWienerKey1 + kPhiloxW1), (kPhiloxM1 * y) ^ (kWienerKey0 + 2u * kPhiloxW0),
+                    __umulhi(kPhiloxM0, s0) ^ (kWienerKey1 + 2u * kPhiloxW1), kPhiloxM0 * s0};
+}
+__device__ __forceinline__ WienerStep wiener_step(uint32_t step, uint32_t id) {
+  const uint32_t x = __umulhi(kPhiloxM1, id) ^ step ^ kWienerKey0;
+  return WienerStep{__umulhi(kPhiloxM0, x), kPhiloxM0 * x};
+}
+__device__ __forceinline__ u32x4 wiener_words(WienerSite p, WienerStep t) {
+  const uint32_t s2 = t.hi ^ p.a;
+  const u32x4 c{__umulhi(kPhiloxM1, s2) ^ p.b, kPhiloxM1 * s2, p.c ^ t.lo, p.d};
+  return philox4x32<7>(c, kWienerKey0 + 3u * kPhiloxW0, kWienerKey1 + 3u * kPhiloxW1);
 }
 
 // Box-Muller, FP32, scaled by s: s (r cos th, r sin th) with r = sqrt(-2 ln u1),

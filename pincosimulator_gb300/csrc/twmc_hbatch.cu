@@ -163,16 +163,18 @@ __device__ __forceinline__ bool hb_next(const StepArgs* __restrict__ pts, const 
 // moves); as a function it is the single system's loop (43 to 48). A CTA that
 // holds whole trajectories copies the arguments to registers first; the
 // cluster splits, with 8 sites per thread more, read them from shared memory.
-// Site-updates/s inlined, by reference, by value: 64x64 4.06, 4.72, 4.67e11;
-// 32x32 3.87, 4.39, 4.76e11; 1x1024 4.85, 5.05e11 (the last two); 16x16 3.46,
-// 3.80e11; 1x32 3.02, 3.10e11; 128x128 3.53, 3.93, 3.70e11.
+// Splits of four slots and more keep the step-independent Philox rounds
+// (WienerSite). Site-updates/s inlined, by reference, by value, and with the
+// rounds kept: 64x64 4.06, 4.72, 4.67, 4.90e11; 32x32 3.87, 4.39, 4.75e11; 16x16
+// 3.46, 3.80, 3.58e11 (by reference, by value, kept); 1x32 3.02, 3.10, 2.97e11
+// (the same); 128x128 3.53, 3.93, 3.70e11, kept by reference 4.45e11.
 template <int V, int NB, bool CH, int CL = 1>
 __device__ __noinline__ void hb_pair(const StepArgs& a, unsigned char* smem_raw, int64_t group) {
   if constexpr (CL == 1) {
     const StepArgs b = a;
-    pair_body<V, NB, CH, PAIR_SCALAR>(b, smem_raw, group);
+    pair_body<V, NB, CH, PAIR_SCALAR, 1, !CH && V * NB >= 4>(b, smem_raw, group);
   } else {
-    pair_body<V, NB, CH, PAIR_SCALAR, CL>(a, smem_raw, group);
+    pair_body<V, NB, CH, PAIR_SCALAR, CL, CL == 4>(a, smem_raw, group);
   }
 }
 

@@ -120,7 +120,9 @@ __host__ __device__ __forceinline__ size_t pair_buffer_bytes(bool chain, int v, 
 // lattice's own two ghost rows among them) through distributed shared
 // memory, so that all loads are local and one cluster barrier separates the
 // writes from the reads.
-template <int V, int NB, bool CH, int PAR, int CL = 1>
+// KEEP: the step-independent part of every pair's Philox rounds stays in registers
+// (WienerSite, four per pair).
+template <int V, int NB, bool CH, int PAR, int CL = 1, bool KEEP = false>
 __device__ __forceinline__ void pair_body(const StepArgs& a, unsigned char* smem_raw, int64_t group) {
   static_assert(CL == 1 || !CH, "chains run on one CTA");
   const int N = int(a.nsites), half = N >> 1;
@@ -182,6 +184,11 @@ __device__ __forceinline__ void pair_body(const StepArgs& a, unsigned char* smem
     }
   }
   const uint32_t seed = a.seeds[tr], id = a.ids[tr];
+  WienerSite ws[KEEP ? NB : 1][KEEP ? V : 1];
+#pragma unroll
+  for (int i = 0; i < (KEEP ? NB : 0); ++i)
+#pragma unroll
+    for (int j = 0; j < V; ++j) ws[i][j] = wiener_site(uint32_t(qr + q0[i] + j * ny), seed, id);
   uint32_t buf = 0;
   if constexpr (CL > 1) {  // every CTA of the cluster is there, and done with what ran before
     cluster_arrive();
@@ -189,6 +196,7 @@ __device__ __forceinline__ void pair_body(const StepArgs& a, unsigned char* smem
   }
   for (int64_t step = 0; step < a.nsteps; ++step) {
     const uint32_t gstep = a.step0 + uint32_t(step);
+    const WienerStep wt = wiener_step(gstep, id);
     const uint32_t cur = base0 + buf;
 #pragma unroll
     for (int i = 0; i < NB; ++i) {
@@ -235,7 +243,10 @@ __device__ __forceinline__ void pair_body(const StepArgs& a, unsigned char* smem
           sx = __fadd2_rn(__fadd2_rn(rt.x, lf.x), sx);
           sy = __fadd2_rn(__fadd2_rn(rt.y, lf.y), sy);
         }
-        const PairNoise nz = pair_noise(wiener_words(uint32_t(q), gstep, seed, id), k.kn);
+        u32x4 w;
+        if constexpr (KEEP) w = wiener_words(ws[i][j], wt);
+        else w = wiener_words(uint32_t(q), gstep, seed, id);
+        const PairNoise nz = pair_noise(w, k.kn);
         up = v[i][j];
         if constexpr (PAR == PAIR_SCALAR) {
           v[i][j] = pair_update(v[i][j], sx, sy, k.ax, k.ay, k.bx, k.by, k.fx, k.fy, k.jt, nz);

@@ -20,14 +20,26 @@ struct PairPlan {
   size_t smem = 0;
 };
 
-// Register caps. 128 registers hold four slots of state (32), the hoisted
-// Philox rounds and the loads in flight without spilling; measured on GB300 at
+// Which 128-register splits keep the step-independent Philox rounds: four
+// products fewer per pair and step against four registers more per pair. GB300,
+// 1e11 site-updates/s without / with: runs of five rows 3.93 / 4.36 (50x50, per-site
+// omega) and 4.00 / 4.30 (scalars); 2 x 2 slots 5.03 / 5.17 (64x64, per-site omega),
+// but 5.32 / 5.23 with scalars; clusters of four 4.15 / 4.25 (128x128, scalars),
+// but 4.24 / 4.16 with per-site omega (120 bytes of spills). One or two slots,
+// chains: the compiler does as well by itself (1x64 2.58 / 2.42).
+constexpr bool pair_keep(int v, int nb, bool ch, int par, int cl) {
+  if (cl > 1) return par == PAIR_SCALAR;
+  return !ch && ((par == PAIR_RSL_IM && v * nb >= 4) || (par == PAIR_SCALAR && v >= 4));
+}
+
+// Register caps. 128 registers hold four slots of state (32), what is kept of
+// the Philox rounds and the loads in flight without spilling; measured on GB300 at
 // 32x32 with 128-thread CTAs, four per SM: 5.55e11 site-updates/s at 128
 // registers, 5.3e11 at 80, 5.1e11 at 64 (144 bytes of spills).
 template <int V, int NB, bool CH, int PAR>
 __global__ void __launch_bounds__(512, 1) pair_kernel(const __grid_constant__ StepArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  pair_body<V, NB, CH, PAR>(a, smem_raw, blockIdx.x);
+  pair_body<V, NB, CH, PAR, 1, pair_keep(V, NB, CH, PAR, 1)>(a, smem_raw, blockIdx.x);
 }
 template <int V, int NB, bool CH, int PAR>
 __global__ void __launch_bounds__(1024, 1) pair_kernel_wide(const __grid_constant__ StepArgs a) {
@@ -37,7 +49,7 @@ __global__ void __launch_bounds__(1024, 1) pair_kernel_wide(const __grid_constan
 template <int V, int CL, int PAR>
 __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(256, 2) pair_cluster_kernel(const __grid_constant__ StepArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  pair_body<V, 1, false, PAR, CL>(a, smem_raw, blockIdx.x / CL);
+  pair_body<V, 1, false, PAR, CL, pair_keep(V, 1, false, PAR, CL)>(a, smem_raw, blockIdx.x / CL);
 }
 template <int V, int CL, int PAR>
 __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(1024, 1) pair_cluster_kernel_wide(const __grid_constant__ StepArgs a) {
