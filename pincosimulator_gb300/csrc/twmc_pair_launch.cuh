@@ -20,13 +20,12 @@ struct PairPlan {
   size_t smem = 0;
 };
 
-// Which 128-register splits keep the step-independent Philox rounds: four
-// products fewer per pair and step against four registers more per pair. GB300,
-// 1e11 site-updates/s without / with: runs of five rows 3.93 / 4.36 (50x50, per-site
+// Which 128-register splits keep the step-independent Philox rounds in registers
+// of their own (WienerSite) instead of as the compiler hoists them. GB300, 1e11 site-updates/s without / with: runs of five rows 3.93 / 4.36 (50x50, per-site
 // omega) and 4.00 / 4.30 (scalars); 2 x 2 slots 5.03 / 5.17 (64x64, per-site omega),
 // but 5.32 / 5.23 with scalars; clusters of four 4.15 / 4.25 (128x128, scalars),
 // but 4.24 / 4.16 with per-site omega (120 bytes of spills). One or two slots,
-// chains: the compiler does as well by itself (1x64 2.58 / 2.42).
+// chains: the compiler does better by itself (1x64 2.58 / 2.42).
 constexpr bool pair_keep(int v, int nb, bool ch, int par, int cl) {
   if (cl > 1) return par == PAIR_SCALAR;
   return !ch && ((par == PAIR_RSL_IM && v * nb >= 4) || (par == PAIR_SCALAR && v >= 4));
