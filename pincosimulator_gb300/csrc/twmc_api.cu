@@ -9,6 +9,7 @@
 #include <cstring>
 #include <limits>
 #include <map>
+#include <memory>
 #include <new>
 #include <string>
 #include <tuple>
@@ -114,6 +115,8 @@ struct twmc_handle {
   // page-locked host staging for fields copied row by row to the caller
   double* h_stage = nullptr;
   size_t h_stage_bytes = 0;
+  // host sources of the uploads since the stream was last waited for
+  std::vector<std::shared_ptr<void>> uploads;
   std::vector<double> ft_times;   // with sentinel
   std::vector<cd> ft_vals, ft_slopes;
   // kernel selection
@@ -171,27 +174,38 @@ void read_matrix(const twmc_matrix& src, int64_t n, Matrix* m) {
 
 size_t rsize(int prec) { return prec ? sizeof(double) : sizeof(float); }
 
-// Uploads go on the handle's stream, in order with the kernels that read them
-// (copies from pageable memory return with the source staged).
+// Uploads go on the handle's stream, in order with the kernels that read them.
+// A copy from pageable memory may return before it has read its source (on a
+// host whose memory the GPU reads coherently nothing need be staged), so the
+// handle keeps the source until the stream has been waited for.
 template <typename T>
-bool upload_raw(DevBuf* b, const T* data, size_t n, cudaStream_t s) {
-  if (!b->ensure(n * sizeof(T))) return false;
-  return cudaMemcpyAsync(b->p, data, n * sizeof(T), cudaMemcpyHostToDevice, s) == cudaSuccess;
+bool upload_raw(twmc_handle* h, DevBuf* b, std::vector<T> v) {
+  const size_t bytes = v.size() * sizeof(T);
+  if (!b->ensure(bytes)) return false;
+  auto kept = std::make_shared<std::vector<T>>(std::move(v));
+  h->uploads.push_back(kept);
+  return cudaMemcpyAsync(b->p, kept->data(), bytes, cudaMemcpyHostToDevice, h->stream) == cudaSuccess;
+}
+
+// Waits for the handle's stream; the sources of its uploads are free then.
+cudaError_t settle(twmc_handle* h) {
+  const cudaError_t e = cudaStreamSynchronize(h->stream);
+  if (e == cudaSuccess) h->uploads.clear();
+  return e;
 }
 
 // Upload complex values in the state precision.
-bool upload_c(DevBuf* b, const std::vector<cd>& v, int prec, cudaStream_t s) {
+bool upload_c(twmc_handle* h, DevBuf* b, std::vector<cd> v) {
   const size_t n = v.size();
-  if (prec) return upload_raw(b, v.data(), n, s);
+  if (h->prec) return upload_raw(h, b, std::move(v));
   std::vector<float> f(2 * n);
   for (size_t i = 0; i < n; ++i) { f[2 * i] = float(v[i].real()); f[2 * i + 1] = float(v[i].imag()); }
-  return upload_raw(b, f.data(), f.size(), s);
+  return upload_raw(h, b, std::move(f));
 }
 
-bool upload_r(DevBuf* b, const std::vector<double>& v, int prec, cudaStream_t s) {
-  if (prec) return upload_raw(b, v.data(), v.size(), s);
-  std::vector<float> f(v.begin(), v.end());
-  return upload_raw(b, f.data(), f.size(), s);
+bool upload_r(twmc_handle* h, DevBuf* b, std::vector<double> v) {
+  if (h->prec) return upload_raw(h, b, std::move(v));
+  return upload_raw(h, b, std::vector<float>(v.begin(), v.end()));
 }
 
 // NoisyMatrix::SetTemporalValue (NoisyMatrix.cpp:164-250).
@@ -302,7 +316,7 @@ int build_tables(twmc_handle* h) {
     std::vector<cd> tw;
     for (int64_t j = 0; j < M0; ++j) tw.push_back(std::polar(1.0, -2.0 * M_PI * double(j) / double(M0)));
     for (int64_t j = 0; j < M1; ++j) tw.push_back(std::polar(1.0, -2.0 * M_PI * double(j) / double(M1)));
-    if (!upload_c(&h->d_tw, tw, prec, h->stream)) return fail(h, TWMC_ERR_NOMEM, "twiddle table upload");
+    if (!upload_c(h, &h->d_tw, std::move(tw))) return fail(h, TWMC_ERR_NOMEM, "twiddle table upload");
     // separable k-space table: [2J fy cos(2 pi ky / ny) / N for ky < M0 |
     // 2J fx cos(2 pi kx / nx) / N for kx < M1]; the kernel adds the two.
     // the FP32 kernel folds dt into the hopping term (local_update_fused)
@@ -311,7 +325,7 @@ int build_tables(twmc_handle* h) {
     std::vector<double> kt;
     for (int64_t k = 0; k < M0; ++k) kt.push_back(scale * fy * std::cos(2.0 * M_PI / double(h->ny) * double(k)));
     for (int64_t k = 0; k < M1; ++k) kt.push_back(scale * fx * std::cos(2.0 * M_PI / double(h->nx) * double(k)));
-    if (!upload_r(&h->d_ktab, kt, prec, h->stream)) return fail(h, TWMC_ERR_NOMEM, "k table upload");
+    if (!upload_r(h, &h->d_ktab, std::move(kt))) return fail(h, TWMC_ERR_NOMEM, "k table upload");
     if (h->integrator == TWMC_INTEGRATOR_SPLIT) {
       // (exp(-i theta) - 1) / N, theta = 2J (fx cos(2 pi kx / nx) + fy cos(2 pi ky / ny)) dt, at every
       // position p of the forward plan's output (frequencies bit-reversed per dimension);
@@ -330,7 +344,7 @@ int build_tables(twmc_handle* h) {
         const double sh = std::sin(0.5 * th);
         kf[size_t(p)] = cd(-2.0 * sh * sh, -std::sin(th)) / double(h->nsites);
       }
-      if (!upload_c(&h->d_kfac, kf, prec, h->stream)) return fail(h, TWMC_ERR_NOMEM, "split-step table upload");
+      if (!upload_c(h, &h->d_kfac, std::move(kf))) return fail(h, TWMC_ERR_NOMEM, "split-step table upload");
     }
   } else if (h->lattice == TWMC_LATTICE_LIEB) {
     // Coupling triplets of TWMCLiebSolver::Setup (TWMCLiebSolver.cpp:54-85).
@@ -370,14 +384,14 @@ int build_tables(twmc_handle* h) {
         else { idx[size_t(c * 4 + j)] = int(c); w[size_t(c * 4 + j)] = cd(0, 0); }
       }
     }
-    if (!upload_raw(&h->d_nbr_idx, idx.data(), idx.size(), h->stream)) return fail(h, TWMC_ERR_NOMEM, "neighbour upload");
-    if (!upload_c(&h->d_nbr_w, w, prec, h->stream)) return fail(h, TWMC_ERR_NOMEM, "neighbour upload");
+    if (!upload_raw(h, &h->d_nbr_idx, std::move(idx))) return fail(h, TWMC_ERR_NOMEM, "neighbour upload");
+    if (!upload_c(h, &h->d_nbr_w, std::move(w))) return fail(h, TWMC_ERR_NOMEM, "neighbour upload");
   }
   if (h->timedep) {
     std::vector<cd> iv(h->ft_vals.size()), is(h->ft_slopes.size());
     for (size_t i = 0; i < iv.size(); ++i) iv[i] = cd(0, 1) * h->ft_vals[i];
     for (size_t i = 0; i < is.size(); ++i) is[i] = cd(0, 1) * h->ft_slopes[i];
-    if (!upload_c(&h->d_ft_vals, iv, prec, h->stream) || !upload_c(&h->d_ft_slopes, is, prec, h->stream))
+    if (!upload_c(h, &h->d_ft_vals, std::move(iv)) || !upload_c(h, &h->d_ft_slopes, std::move(is)))
       return fail(h, TWMC_ERR_NOMEM, "F(t) table upload");
   }
   // the matrices of the initial draws, the same for every batch of the handle
@@ -385,7 +399,7 @@ int build_tables(twmc_handle* h) {
   {
     const Matrix* mats[3] = {&h->m_U, &h->m_omega, &h->m_F};
     auto up = [&](DevBuf* b, const std::vector<cd>& v) {
-      return upload_raw(b, reinterpret_cast<const double*>(v.data()), 2 * v.size(), h->stream);
+      return upload_raw(h, b, v);
     };
     bool ok = (h->m_binit.base_uniform() || up(&h->d_binit, h->m_binit.base)) &&
               (h->m_bsigma.base_uniform() || up(&h->d_bsigma, h->m_bsigma.base));
@@ -408,8 +422,9 @@ int build_tables(twmc_handle* h) {
         v[size_t(p)] = cd(-x.imag(), x.real());
       }
     }
-    if (!upload_c(&h->d_shared_par[k], v, prec, h->stream)) return fail(h, TWMC_ERR_NOMEM, "parameter upload");
+    if (!upload_c(h, &h->d_shared_par[k], std::move(v))) return fail(h, TWMC_ERR_NOMEM, "parameter upload");
   }
+  TWMC_CUDA(h, settle(h));
   return TWMC_OK;
 }
 
@@ -552,6 +567,7 @@ int reduce(twmc_handle* h) {
 int batch_init(twmc_handle* h, const twmc_task_desc* tasks, size_t n, const bool (&want_real)[3]) {
   const int64_t N = h->nsites;
   const int prec = h->prec;
+  if (!h->uploads.empty()) TWMC_CUDA(h, settle(h));  // (a batch that nothing has waited for)
   h->ntraj = int64_t(n);
   h->step_pos = 0;
   const size_t c2 = 2 * rsize(prec);
@@ -573,7 +589,7 @@ int batch_init(twmc_handle* h, const twmc_task_desc* tasks, size_t n, const bool
     ids[i] = uint32_t(tasks[i].id);
     if (tasks[i].ic_kind != ic) return fail(h, TWMC_ERR_INVALID, "tasks of one batch must share ic_kind");
   }
-  if (!upload_raw(&h->d_seeds, seeds.data(), n, h->stream) || !upload_raw(&h->d_ids, ids.data(), n, h->stream))
+  if (!upload_raw(h, &h->d_seeds, std::move(seeds)) || !upload_raw(h, &h->d_ids, std::move(ids)))
     return fail(h, TWMC_ERR_NOMEM, "seed upload");
   InitArgs ia;
   std::memset(&ia, 0, sizeof(ia));
@@ -600,7 +616,7 @@ int batch_init(twmc_handle* h, const twmc_task_desc* tasks, size_t n, const bool
       if (!tasks[i].init_field) return fail(h, TWMC_ERR_INVALID, "TWMC_IC_GIVEN task without init_field");
       std::memcpy(&g[size_t(2 * N) * i], tasks[i].init_field, sizeof(double) * size_t(2 * N));
     }
-    if (!upload_raw(&h->d_given, g.data(), g.size(), h->stream)) return fail(h, TWMC_ERR_NOMEM, "initial field upload");
+    if (!upload_raw(h, &h->d_given, std::move(g))) return fail(h, TWMC_ERR_NOMEM, "initial field upload");
     ia.given = h->d_given.as<double>();
   }
   // Real part of rsl = Im(omega) - gamma/2 (Lieb: -Im(E) - gamma/2), and of
@@ -638,7 +654,7 @@ int batch_init(twmc_handle* h, const twmc_task_desc* tasks, size_t n, const bool
         if (!src) return fail(h, TWMC_ERR_INVALID, "disorder realisations must be given for all tasks of a batch or none");
         std::memcpy(&g[size_t(2 * N) * i], src, sizeof(double) * size_t(2 * N));
       }
-      if (!upload_raw(&h->d_given_real[m], g.data(), g.size(), h->stream)) return fail(h, TWMC_ERR_NOMEM, "realisation upload");
+      if (!upload_raw(h, &h->d_given_real[m], std::move(g))) return fail(h, TWMC_ERR_NOMEM, "realisation upload");
       ia.given_real[m] = h->d_given_real[m].as<double>();
     }
   }
@@ -959,7 +975,7 @@ int twmc_batch_reduce(twmc_handle* h) {
 int twmc_sync(twmc_handle* h, double* kernel_ms) {
   if (!h) return TWMC_ERR_INVALID;
   cudaSetDevice(h->device);
-  cudaError_t e = cudaStreamSynchronize(h->stream);
+  cudaError_t e = settle(h);
   if (e != cudaSuccess) return cuda_fail(h, e, "cudaStreamSynchronize");
   double ms = h->carry_ms;  // step launches of twmc_run calls since the last twmc_sync
   h->carry_ms = 0.0;
@@ -1054,7 +1070,7 @@ int twmc_run(twmc_handle* h, const twmc_task_desc* tasks, size_t n, twmc_outputs
           return fail(h, TWMC_ERR_INVALID, "noise buffer must hold n_tasks x steps x n_sites values (one task group)");
         std::vector<cd> nz(need);
         for (size_t i = 0; i < need; ++i) nz[i] = cd(h->noise_host[2 * i], h->noise_host[2 * i + 1]);
-        if (!upload_c(&h->d_noise, nz, h->prec, h->stream)) return fail(h, TWMC_ERR_NOMEM, "noise upload");
+        if (!upload_c(h, &h->d_noise, std::move(nz))) return fail(h, TWMC_ERR_NOMEM, "noise upload");
         h->noise_steps = s.steps;
       }
       if (h->timedep) {
@@ -1068,8 +1084,8 @@ int twmc_run(twmc_handle* h, const twmc_task_desc* tasks, size_t n, twmc_outputs
           hint = seg.first;
         }
         std::vector<float> offs_f(offs.begin(), offs.end());
-        if (!upload_raw(&h->d_ft_id, ids.data(), ids.size(), h->stream) || !upload_raw(&h->d_ft_dt, offs.data(), offs.size(), h->stream) ||
-            !upload_raw(&h->d_ft_dt_f, offs_f.data(), offs_f.size(), h->stream))
+        if (!upload_raw(h, &h->d_ft_id, std::move(ids)) || !upload_raw(h, &h->d_ft_dt, std::move(offs)) ||
+            !upload_raw(h, &h->d_ft_dt_f, std::move(offs_f)))
           return fail(h, TWMC_ERR_NOMEM, "F(t) schedule upload");
       }
       // realisations of noisy matrices
@@ -1288,7 +1304,7 @@ int twmc_run(twmc_handle* h, const twmc_task_desc* tasks, size_t n, twmc_outputs
       }
       std::vector<int> st(bn);
       TWMC_CUDA(h, cudaMemcpyAsync(st.data(), h->d_status.p, bn * sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-      TWMC_CUDA(h, cudaStreamSynchronize(h->stream));
+      TWMC_CUDA(h, settle(h));
       if (dl_used) TWMC_CUDA(h, cudaStreamSynchronize(h->dl_stream));
       for (size_t i = 0; i < bn; ++i) {
         if (out && out->status) out->status[idx[i]] = st[i];

@@ -1,0 +1,83 @@
+"""Host code of the library on the CPU, linked with a stand-in for the CUDA
+runtime (fake_cudart.cpp) whose streams run their work as late as the runtime
+allows. Each test runs a script in a process of its own."""
+import glob
+import os
+import subprocess
+import sys
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+ROOT = os.path.dirname(HERE)
+PRELUDE = """
+import ctypes as C
+import numpy as np
+from pincosimulator_gb300 import twmc
+lib = twmc.load()
+for f in ("fake_uploads", "fake_changed", "fake_lowered"):
+    getattr(lib, f).restype = C.c_long
+lib.fake_pinned_peak.restype = C.c_size_t
+lib.fake_pinned_limit.argtypes = [C.c_size_t]
+lib.fake_fail_launch.argtypes = [C.c_char_p, C.c_long]
+lib.fake_log.restype = C.c_char_p
+"""
+
+
+@pytest.fixture(scope="session")
+def fake_lib(built_lib, tmp_path_factory):
+    d = tmp_path_factory.mktemp("fake_cudart")
+    obj, lib = str(d / "fake.o"), str(d / "libtwmc_fake.so")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-fPIC", "-I/usr/local/cuda/include", "-c",
+                    os.path.join(HERE, "fake_cudart.cpp"), "-o", obj], check=True)
+    from pincosimulator_gb300 import build_ext
+
+    objs = [os.path.join(build_ext.BUILD, s.replace(".cu", ".o")) for s in build_ext.SOURCES]
+    subprocess.run(["g++", "-shared", "-Wl,-Bsymbolic", "-Wl,--no-undefined", *objs, obj, "-o", lib], check=True)
+    return lib
+
+
+@pytest.fixture
+def script(fake_lib):
+    def go(text):
+        r = subprocess.run([sys.executable, "-c", PRELUDE + text], capture_output=True, text=True, timeout=120,
+                           env=dict(os.environ, TWMC_LIB=fake_lib, PYTHONPATH=ROOT))
+        assert r.returncode == 0, r.stdout + r.stderr
+        return r.stdout
+    return go
+
+
+def test_sources_of_uploads_live_until_their_copies_have_run(script):
+    """An asynchronous copy from pageable memory may read its source after the
+    call: tables, parameters, seeds, given fields and realisations, caller noise
+    and the F(t) schedule must still be there when the stream runs it."""
+    script("""
+rng = np.random.default_rng(1)
+c = lambda *s: rng.normal(size=s) + 1j * rng.normal(size=s)
+def square(n_traj=5, **kw):
+    a = dict(nx=16, ny=16, J=1.0, dt=0.01, frame_steps=2, omega=c(256), U=twmc.Noisy(c(256), 1, c(256)), F=c(256),
+             beta_init=c(256), beta_init_sigma=c(256))
+    a.update(kw)
+    s = twmc.System(**a)
+    t = s.make_tasks(n_traj, t_end=0.04, ic=twmc.IC_GIVEN, init_field=c(n_traj, 256),
+                     realizations={"U": c(n_traj, 256)})
+    return s, t
+for prec in (twmc.PREC_F32, twmc.PREC_F64):
+    for integ in (twmc.INTEGRATOR_EULER, twmc.INTEGRATOR_SPLIT):
+        s, t = square(precision=prec, integrator=integ)
+        s.run(t, realizations=True)
+        s.run(t, moments=True)
+        s.batch_init(t); s.advance(3); s.batch_init(t); s.advance(3); s.reduce(); s.sync()
+        s.close()
+    s, t = square(precision=prec, noise=twmc.NOISE_BUFFER)
+    s.set_noise(c(5, 4, 256))
+    s.run(t)
+    s.close()
+    times = np.arange(0, 0.1, 0.01)
+    s = twmc.System(lattice=twmc.LATTICE_LIEB, nx=1, ny=8, J_AB=1.0, J_BC=1.0, dt=0.002, frame_steps=5, precision=prec,
+                    U=c(24), F_t=(times, c(len(times), 24)))
+    s.run(s.make_tasks(3, t_end=0.04))
+    s.close()
+assert lib.fake_uploads() > 60, lib.fake_uploads()
+assert lib.fake_changed() == 0, (lib.fake_changed(), lib.fake_uploads())
+""")
