@@ -30,8 +30,12 @@
 #include <vector>
 
 #include "twmc.h"
+#include "twmc_mlp_map.h"
 
 namespace {
+
+using twmc::LayerMap;
+using twmc::weight_slot;
 
 using bf16 = __nv_bfloat16;
 
@@ -276,14 +280,6 @@ __global__ void cast_input_kernel(const float* __restrict__ x, int64_t rows, int
     y[(i / cols) * ld + i % cols] = __float2bfloat16(x[i]);
 }
 
-// Where the layers' parameters lie: W_l [n][k] and then b_l [n] at `off` of the
-// FP32 arrays, the BF16 copy of W_l at `h`, ld apart.
-constexpr int kMaxLayers = 16;
-struct LayerMap {
-  int64_t off[kMaxLayers], h[kMaxLayers];
-  int n[kMaxLayers], k[kMaxLayers], ld[kMaxLayers];
-};
-
 // The BF16 copy of every layer's weights: grid (rows, layer).
 __global__ void cast_params_kernel(const float* __restrict__ w, bf16* __restrict__ w16, const __grid_constant__ LayerMap m) {
   const int l = blockIdx.y, K = m.k[l];
@@ -334,8 +330,8 @@ __global__ void adam_kernel(float* __restrict__ w, bf16* __restrict__ w16, const
     for (int c = 0; c < 4; ++c) {
       if (c >= cnt) break;
       if (l + 1 < nl && i + c >= lm.off[l + 1]) ++l;
-      const uint32_t at = uint32_t(i + c - lm.off[l]), r = at / uint32_t(lm.k[l]);
-      if (r < uint32_t(lm.n[l])) w16[lm.h[l] + int64_t(r) * lm.ld[l] + (at - r * uint32_t(lm.k[l]))] = __float2bfloat16(wv[c]);
+      const int64_t slot = weight_slot(lm, l, i + c);
+      if (slot >= 0) w16[slot] = __float2bfloat16(wv[c]);
     }
   }
 }
