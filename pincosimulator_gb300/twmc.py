@@ -77,7 +77,11 @@ def _most_frames(tasks, dt_obs: float) -> int:
         return t[:, f.offset:f.offset + f.size].copy().view(dtype)[:, 0]
 
     span = (field(TaskDesc.t_end, np.float64) - field(TaskDesc.t_start, np.float64)) / dt_obs
-    return int((np.rint(span).astype(np.int64) + field(TaskDesc.store_initial, np.int32)).max())
+    store = field(TaskDesc.store_initial, np.int32)
+    finite = np.isfinite(span)
+    # the largest count, or the first span that is not finite, which round() refuses
+    i = int(np.argmax(np.rint(span) + store)) if finite.all() else int(np.argmin(finite))
+    return int(round(float(span[i]))) + int(store[i])
 
 
 class PointDesc(C.Structure):
