@@ -704,6 +704,7 @@ int download_real(twmc_handle* h, const DevBuf& b, double* out, size_t n) {
 constexpr size_t kWideChunk = size_t(1) << 25;  // 256 MB of doubles
 constexpr int kFinalChunks = 4;                  // trajectory ranges of the final-field pipeline
 constexpr size_t kCollectMax = size_t(1) << 28;  // most bytes of frames collected on the device
+constexpr size_t kStagePiece = size_t(1) << 24;  // page-locked bytes they go home through
 constexpr size_t kSnapMax = size_t(8) << 30;     // largest final field (bytes) the pipeline stages
 
 // m device rows of `row` doubles (consecutive) to host rows `row_stride`
@@ -777,23 +778,34 @@ int download_scatter(twmc_handle* h, Dst dst) {
 }
 
 // The collected frames (rows of `row` doubles in d_frames) to the caller's rows:
-// straight into page-locked memory, else through the handle's page-locked
-// buffer.
+// straight into page-locked memory, else in pieces through the handle's
+// page-locked buffer, as large as the largest single frame of these runs,
+// or straight into pageable memory where there is none to be had.
 int download_collected(twmc_handle* h, double* out, size_t row_stride, size_t row, size_t rows) {
-  cudaPointerAttributes at;
-  const bool locked = cudaPointerGetAttributes(&at, out) == cudaSuccess && at.type == cudaMemoryTypeHost;
-  cudaGetLastError();
-  if (locked) {
+  const size_t total = rows * row, piece = std::min(total, kStagePiece / sizeof(double));
+  auto locked = [](const double* p) {
+    cudaPointerAttributes at;
+    const bool yes = cudaPointerGetAttributes(&at, p) == cudaSuccess && at.type == cudaMemoryTypeHost;
+    cudaGetLastError();
+    return yes;
+  };
+  if ((locked(out) && locked(out + (rows - 1) * row_stride + row - 1)) || ensure_stage(h, piece * sizeof(double)) != TWMC_OK) {
+    cudaGetLastError();
+    h->err.clear();
     TWMC_CUDA(h, copy_rows_d2h(h->device, out, row_stride, h->d_frames.p, row, rows, h->stream));
     return TWMC_OK;
   }
-  const size_t bytes = rows * row * sizeof(double);
-  int rc = ensure_stage(h, bytes);
-  if (rc) return rc;
-  TWMC_CUDA(h, cudaMemcpyAsync(h->h_stage, h->d_frames.p, bytes, cudaMemcpyDeviceToHost, h->stream));
-  TWMC_CUDA(h, cudaStreamSynchronize(h->stream));
-  if (row_stride == row) std::memcpy(out, h->h_stage, bytes);
-  else for (size_t r = 0; r < rows; ++r) std::memcpy(out + r * row_stride, h->h_stage + r * row, row * sizeof(double));
+  for (size_t o = 0; o < total; o += piece) {
+    const size_t end = std::min(o + piece, total);
+    TWMC_CUDA(h, cudaMemcpyAsync(h->h_stage, h->d_frames.as<double>() + o, (end - o) * sizeof(double),
+                                 cudaMemcpyDeviceToHost, h->stream));
+    TWMC_CUDA(h, cudaStreamSynchronize(h->stream));
+    for (size_t k = o; k < end;) {  // whole or part rows
+      const size_t m = row_stride == row ? end - k : std::min(end - k, row - k % row);
+      std::memcpy(out + (k / row) * row_stride + k % row, h->h_stage + (k - o), m * sizeof(double));
+      k += m;
+    }
+  }
   return TWMC_OK;
 }
 

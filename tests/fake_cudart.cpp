@@ -76,6 +76,7 @@ long fake_changed() { return g_changed; }           // of those, with another so
 long fake_lowered() { return g_lowered; }           // dynamic shared-memory limits set below an earlier value
 size_t fake_pinned_peak() { return pinned_peak; }
 void fake_pinned_limit(size_t n) { pinned_limit = n; pinned_peak = pinned_now; }
+void fake_pin(void* p, size_t n) { pinned()[static_cast<char*>(p)] = n; }  // as cudaHostRegister
 void fake_fail_launch(const char* name, long nth) { g_fail_name = name; g_fail_at = nth; }  // the nth of that name from now on
 void fake_hook(void (*f)(const char*)) { g_hook = f; }  // called as each kernel runs
 const char* fake_log() { return g_log.c_str(); }
@@ -129,6 +130,10 @@ cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) {
   return cudaSuccess;
 }
 cudaError_t cudaEventSynchronize(cudaEvent_t e) { auto* p = reinterpret_cast<Event*>(e); if (p->s) drain(p->s, p->at); return cudaSuccess; }
+cudaError_t cudaEventQuery(cudaEvent_t e) {
+  auto* p = reinterpret_cast<Event*>(e);
+  return !p->s || p->s->done >= p->at ? cudaSuccess : ret(cudaErrorNotReady);
+}
 cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t) { *ms = 1.0f; return cudaSuccess; }
 cudaError_t cudaStreamWaitEvent(cudaStream_t s, cudaEvent_t e, unsigned) {
   const Event v = *reinterpret_cast<Event*>(e);
@@ -159,6 +164,8 @@ cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void* p) {
   return cudaSuccess;
 }
 cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind k, cudaStream_t st) {
+  const char* host = static_cast<const char*>(k == cudaMemcpyHostToDevice ? s : d);
+  if (n && k != cudaMemcpyDeviceToDevice && is_pinned(host) != is_pinned(host + n - 1)) return ret(cudaErrorInvalidValue);
   if (k == cudaMemcpyHostToDevice && !is_pinned(s)) {
     std::string was(static_cast<const char*>(s), n);
     push(of(st), [=] {

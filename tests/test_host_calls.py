@@ -21,6 +21,11 @@ lib.fake_pinned_peak.restype = C.c_size_t
 lib.fake_pinned_limit.argtypes = [C.c_size_t]
 lib.fake_fail_launch.argtypes = [C.c_char_p, C.c_long]
 lib.fake_log.restype = C.c_char_p
+lib.fake_pin.argtypes = [C.c_void_p, C.c_size_t]
+def chain(n_traj, n_frames, sites=64):
+    s = twmc.System(nx=1, ny=sites, J=1.0, dt=0.01, frame_steps=2, omega=-0.5, U=0.2, F=1.0, beta_init_sigma=0.5)
+    t = s.make_tasks(n_traj, t_end=0.02 * (n_frames - 1))
+    return s, t, {"frames": np.full((n_traj, n_frames, sites), np.nan + 0j)}
 """
 
 
@@ -80,4 +85,35 @@ for prec in (twmc.PREC_F32, twmc.PREC_F64):
     s.close()
 assert lib.fake_uploads() > 60, lib.fake_uploads()
 assert lib.fake_changed() == 0, (lib.fake_changed(), lib.fake_uploads())
+""")
+
+
+def test_collected_frames_without_page_locked_memory(script):
+    """The buffer that frames go home through is bounded, and a run does
+    not need it."""
+    script("""
+s, t, bufs = chain(500, 80)   # 41 MB of frames
+s.run(t, buffers=bufs)
+assert not np.isnan(bufs["frames"]).any()
+assert 0 < lib.fake_pinned_peak() <= 1 << 24, lib.fake_pinned_peak()
+s.close()
+for limit in (0, 1 << 20):
+    lib.fake_pinned_limit(limit)
+    s, t, bufs = chain(500, 8)   # 4 MB
+    s.run(t, buffers=bufs)
+    assert not np.isnan(bufs["frames"]).any()
+    s.close()
+""")
+
+
+def test_partly_page_locked_frames(script):
+    """A caller's array of which only a part is page-locked: not one copy, which
+    the runtime refuses."""
+    script("""
+for part in (4096, 100000):
+    s, t, bufs = chain(20, 10)
+    lib.fake_pin(bufs["frames"].ctypes.data, part)
+    s.run(t, buffers=bufs)
+    assert not np.isnan(bufs["frames"]).any()
+    s.close()
 """)
