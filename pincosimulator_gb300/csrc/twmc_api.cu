@@ -7,6 +7,7 @@
 #include <cmath>
 #include <complex>
 #include <cstring>
+#include <functional>
 #include <limits>
 #include <map>
 #include <memory>
@@ -1140,6 +1141,18 @@ int twmc_run(twmc_handle* h, const twmc_task_desc* tasks, size_t n, twmc_outputs
         }
       } drain{h};
       const size_t row = size_t(2 * N);  // doubles per trajectory
+      // The frames placed so far reach the caller also when the run ends early
+      // (declared after `drain`: runs before it).
+      int64_t placed = 0;
+      struct OnExit {
+        std::function<void()> f;
+        ~OnExit() { f(); }
+      } flush{[&] {
+        if (!collect || placed == 0) return;
+        const size_t rows_d = size_t(s.n_frames) * row * sizeof(double), rows_h = size_t(max_frames) * row * sizeof(double);
+        cudaMemcpy2DAsync(out->frames + idx[0] * size_t(max_frames) * row, rows_h, h->d_frames.p, rows_d,
+                          size_t(placed) * row * sizeof(double), bn, cudaMemcpyDeviceToHost, h->stream);
+      }};
       auto stage_setup = [&]() -> int {
         if (!h->dl_stream) TWMC_CUDA(h, cudaStreamCreateWithFlags(&h->dl_stream, cudaStreamNonBlocking));
         while (h->dl_ev.size() < size_t(kFinalChunks)) {
@@ -1256,6 +1269,7 @@ int twmc_run(twmc_handle* h, const twmc_task_desc* tasks, size_t n, twmc_outputs
             if (!place_launch(h->prec, h->d_state.p, h->d_frames.as<double>() + size_t(f) * row, int64_t(bn), int64_t(row),
                               int64_t(size_t(s.n_frames) * row), h->stream, &err))
               return fail(h, TWMC_ERR_CUDA, err);
+            placed = f + 1;
           } else {
             int r2 = download_scatter(h, [&](size_t i) { return out->frames + (idx[i] * max_frames + f) * N * 2; });
             if (r2) return r2;
@@ -1313,6 +1327,7 @@ int twmc_run(twmc_handle* h, const twmc_task_desc* tasks, size_t n, twmc_outputs
         rc = download_collected(h, out->frames + idx[0] * size_t(max_frames) * row, size_t(max_frames) * row,
                                 size_t(s.n_frames) * row, bn);
         if (rc) return rc;
+        placed = 0;
       }
       std::vector<int> st(bn);
       TWMC_CUDA(h, cudaMemcpyAsync(st.data(), h->d_status.p, bn * sizeof(int), cudaMemcpyDeviceToHost, h->stream));

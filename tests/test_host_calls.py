@@ -117,3 +117,18 @@ for part in (4096, 100000):
     assert not np.isnan(bufs["frames"]).any()
     s.close()
 """)
+
+
+def test_frames_before_an_error_reach_the_caller(script):
+    script("""
+s, t, bufs = chain(20, 10)
+lib.fake_fail_launch(b"square_fft_kernel", 3)   # the fourth launch: frames 0 to 3 are there
+try:
+    s.run(t, buffers=bufs)
+    raise SystemExit("no error")
+except twmc.TWMCError:
+    pass
+lost = np.isnan(bufs["frames"]).any(axis=(0, 2))
+assert not lost[:4].any() and lost[4:].all(), lost
+s.close()
+""")
