@@ -781,8 +781,10 @@ int download_scatter(twmc_handle* h, Dst dst) {
 // The collected frames (rows of `row` doubles in d_frames) to the caller's rows:
 // straight into page-locked memory, else in pieces through the handle's
 // page-locked buffer, as large as the largest single frame of these runs,
-// or straight into pageable memory where there is none to be had.
-int download_collected(twmc_handle* h, double* out, size_t row_stride, size_t row, size_t rows) {
+// or straight into pageable memory where there is none to be had. wait():
+// called once the first copy is on its way.
+template <typename Wait>
+int download_collected(twmc_handle* h, double* out, size_t row_stride, size_t row, size_t rows, Wait wait) {
   const size_t total = rows * row, piece = std::min(total, kStagePiece / sizeof(double));
   auto locked = [](const double* p) {
     cudaPointerAttributes at;
@@ -794,12 +796,14 @@ int download_collected(twmc_handle* h, double* out, size_t row_stride, size_t ro
     cudaGetLastError();
     h->err.clear();
     TWMC_CUDA(h, copy_rows_d2h(h->device, out, row_stride, h->d_frames.p, row, rows, h->stream));
+    wait();
     return TWMC_OK;
   }
   for (size_t o = 0; o < total; o += piece) {
     const size_t end = std::min(o + piece, total);
     TWMC_CUDA(h, cudaMemcpyAsync(h->h_stage, h->d_frames.as<double>() + o, (end - o) * sizeof(double),
                                  cudaMemcpyDeviceToHost, h->stream));
+    if (o == 0) wait();
     TWMC_CUDA(h, cudaStreamSynchronize(h->stream));
     for (size_t k = o; k < end;) {  // whole or part rows
       const size_t m = row_stride == row ? end - k : std::min(end - k, row - k % row);
@@ -1153,6 +1157,18 @@ int twmc_run(twmc_handle* h, const twmc_task_desc* tasks, size_t n, twmc_outputs
         cudaMemcpy2DAsync(out->frames + idx[0] * size_t(max_frames) * row, rows_h, h->d_frames.p, rows_d,
                           size_t(placed) * row * sizeof(double), bn, cudaMemcpyDeviceToHost, h->stream);
       }};
+      // Progress counts steps that have run: their launches' end events, looked
+      // at after each frame is queued and waited for in order at the end.
+      std::vector<std::pair<cudaEvent_t, double>> marks;
+      size_t marks_seen = 0;
+      auto mark = [&] { marks.push_back({h->ev_pending.back().second, total_steps ? double(done_steps) / double(total_steps) : 1.0}); };
+      auto look = [&](bool wait) {
+        for (; marks_seen < marks.size(); ++marks_seen) {
+          const cudaError_t e = wait ? cudaEventSynchronize(marks[marks_seen].first) : cudaEventQuery(marks[marks_seen].first);
+          if (e != cudaSuccess) { if (e == cudaErrorNotReady) cudaGetLastError(); break; }
+          h->progress = marks[marks_seen].second;
+        }
+      };
       auto stage_setup = [&]() -> int {
         if (!h->dl_stream) TWMC_CUDA(h, cudaStreamCreateWithFlags(&h->dl_stream, cudaStreamNonBlocking));
         while (h->dl_ev.size() < size_t(kFinalChunks)) {
@@ -1305,14 +1321,16 @@ int twmc_run(twmc_handle* h, const twmc_task_desc* tasks, size_t n, twmc_outputs
         if (rc) return rc;
         done_steps += (ss - cur) * int64_t(bn);
         cur = ss;
+        mark();
         rc = save_frame(f++);
         if (rc) return rc;
-        h->progress = total_steps ? double(done_steps) / double(total_steps) : 1.0;
+        look(false);
       }
       if (s.steps > cur) {
         rc = step(s.steps - cur, false, true, nullptr);
         if (rc) return rc;
         done_steps += (s.steps - cur) * int64_t(bn);
+        mark();
       }
       if (out && out->final_field && !final_sent) {  // (a pipelined run has sent it already)
         if (contiguous) {
@@ -1325,12 +1343,13 @@ int twmc_run(twmc_handle* h, const twmc_task_desc* tasks, size_t n, twmc_outputs
       }
       if (collect) {
         rc = download_collected(h, out->frames + idx[0] * size_t(max_frames) * row, size_t(max_frames) * row,
-                                size_t(s.n_frames) * row, bn);
+                                size_t(s.n_frames) * row, bn, [&] { look(true); });
         if (rc) return rc;
         placed = 0;
       }
       std::vector<int> st(bn);
       TWMC_CUDA(h, cudaMemcpyAsync(st.data(), h->d_status.p, bn * sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+      look(true);
       TWMC_CUDA(h, settle(h));
       if (dl_used) TWMC_CUDA(h, cudaStreamSynchronize(h->dl_stream));
       for (size_t i = 0; i < bn; ++i) {

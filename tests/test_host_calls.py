@@ -88,6 +88,31 @@ assert lib.fake_changed() == 0, (lib.fake_changed(), lib.fake_uploads())
 """)
 
 
+@pytest.mark.parametrize("sites", [64, 8192])  # frames collected on the device; frames staged one by one
+def test_progress_counts_steps_that_have_run(script, sites):
+    """At the k-th step launch of a run of five, at most k of them have run."""
+    script(f"sites = {sites}" + """
+s, t, bufs = chain(130, 6, sites)
+seen = []
+def hook(name):
+    if b"fft_kernel" in name or b"pair" in name:
+        p = C.c_double()
+        lib.twmc_progress(s.h, C.byref(p))
+        seen.append(p.value)
+CB = C.CFUNCTYPE(None, C.c_char_p)
+cb = CB(hook)
+lib.fake_hook(cb)
+s.run(t, final=False, buffers=bufs)
+assert len(seen) == 5, seen
+assert all(p <= k / 5 + 1e-12 for k, p in enumerate(seen)), seen
+p = C.c_double()
+lib.twmc_progress(s.h, C.byref(p))
+assert p.value == 1.0
+lib.fake_hook(CB(0))
+s.close()
+""")
+
+
 def test_collected_frames_without_page_locked_memory(script):
     """The buffer that frames go home through is bounded, and a run does
     not need it."""
