@@ -200,7 +200,8 @@ TWMC_API int twmc_batch_advance(twmc_handle* h, int64_t n_steps);
 TWMC_API int twmc_batch_reduce(twmc_handle* h);
 /* Waits for the handle's stream; *kernel_ms = summed device time of the
  * trajectory-step launches since the last call (may be NULL), including those
- * of twmc_run calls made since then. */
+ * of twmc_run calls made since then; launches that run side by side (the
+ * trajectory ranges of a run's last steps) count once. */
 TWMC_API int twmc_sync(twmc_handle* h, double* kernel_ms);
 /* Copies the batch state (n x n_sites complex128) and/or the last moment
  * blocks (n_moment_blocks x n_sites x 3) to host memory; NULL skips. */

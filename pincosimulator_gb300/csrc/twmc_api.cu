@@ -82,6 +82,14 @@ int ilog2_exact(int64_t v) {
 
 }  // namespace
 
+// Timing of one stretch of steps: from `first`, recorded before its launches, to
+// the last of `ends`, one behind each launch (several on streams of their own
+// for a run's last steps).
+struct StepTime {
+  cudaEvent_t first = nullptr;
+  std::vector<cudaEvent_t> ends;
+};
+
 struct twmc_handle {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -139,8 +147,8 @@ struct twmc_handle {
   std::vector<double> noise_host;  // deterministic noise buffer (complex, interleaved)
   bool noise_set = false;
   // timing / counters
-  std::vector<std::pair<cudaEvent_t, cudaEvent_t>> ev_pending;
-  std::vector<std::pair<cudaEvent_t, cudaEvent_t>> ev_free;
+  std::vector<StepTime> ev_pending;
+  std::vector<cudaEvent_t> ev_free;
   int64_t launches = 0;
   double carry_ms = 0.0;  // step-kernel device time of the last twmc_run, not yet reported
   double progress = 0.0;
@@ -429,19 +437,27 @@ int build_tables(twmc_handle* h) {
   return TWMC_OK;
 }
 
-std::pair<cudaEvent_t, cudaEvent_t> get_events(twmc_handle* h) {
-  if (!h->ev_free.empty()) { auto e = h->ev_free.back(); h->ev_free.pop_back(); return e; }
-  cudaEvent_t a, b;
-  cudaEventCreate(&a);
-  cudaEventCreate(&b);
-  return {a, b};
+cudaEvent_t get_event(twmc_handle* h) {
+  cudaEvent_t e = nullptr;
+  if (h->ev_free.empty()) cudaEventCreate(&e);
+  else { e = h->ev_free.back(); h->ev_free.pop_back(); }
+  return e;
+}
+void put_events(twmc_handle* h, const StepTime& t) {
+  h->ev_free.push_back(t.first);
+  h->ev_free.insert(h->ev_free.end(), t.ends.begin(), t.ends.end());
+}
+
+void start_timing(twmc_handle* h) {
+  h->ev_pending.push_back({get_event(h), {}});
+  cudaEventRecord(h->ev_pending.back().first, h->stream);
 }
 
 // Advances the batch by n steps (n may be 0 to refresh the k-space buffer).
 // n steps of trajectories [t0, t1) of the batch (all when t1 < 0); the
-// step counter advances, and the launch is timed, only when `range_stream` is
-// null (a caller stepping the batch in ranges on streams of their own does
-// both once).
+// step counter advances, and the stretch's timing starts, only when
+// `range_stream` is null (a caller stepping the batch in ranges on streams of
+// their own does both once); the launch's end is added to the last stretch.
 int advance(twmc_handle* h, int64_t n, bool want_nk, int64_t t0 = 0, int64_t t1 = -1,
             cudaStream_t range_stream = nullptr) {
   const cudaStream_t stream = range_stream ? range_stream : h->stream;
@@ -521,11 +537,7 @@ int advance(twmc_handle* h, int64_t n, bool want_nk, int64_t t0 = 0, int64_t t1 
     return fail(h, TWMC_ERR_INVALID, "noise buffer shorter than the run");
   int nparams = 0;
   for (int k = 0; k < 3; ++k) nparams += (*par[k] != nullptr);
-  std::pair<cudaEvent_t, cudaEvent_t> ev{nullptr, nullptr};
-  if (!range_stream) {
-    ev = get_events(h);
-    cudaEventRecord(ev.first, stream);
-  }
+  if (!range_stream) start_timing(h);
   std::string err;
   bool ok;
   if (h->use_fft) {
@@ -538,10 +550,8 @@ int advance(twmc_handle* h, int64_t n, bool want_nk, int64_t t0 = 0, int64_t t1 
                std::strcmp(h->last_info.name, "rowrun_kernel") == 0))
       h->kname = h->last_info.name;
   }
-  if (!range_stream) {
-    cudaEventRecord(ev.second, stream);
-    h->ev_pending.push_back(ev);
-  }
+  h->ev_pending.back().ends.push_back(get_event(h));
+  cudaEventRecord(h->ev_pending.back().ends.back(), stream);
   if (!ok) return fail(h, TWMC_ERR_CUDA, err);
   ++h->launches;
   if (!range_stream) h->step_pos += uint32_t(n);
@@ -956,8 +966,8 @@ void twmc_destroy(twmc_handle* h) {
   if (h->snap_free) cudaEventDestroy(h->snap_free);
   for (cudaStream_t s : h->range_stream) cudaStreamDestroy(s);
   if (h->dl_stream) cudaStreamDestroy(h->dl_stream);
-  for (auto& e : h->ev_pending) { cudaEventDestroy(e.first); cudaEventDestroy(e.second); }
-  for (auto& e : h->ev_free) { cudaEventDestroy(e.first); cudaEventDestroy(e.second); }
+  for (const StepTime& t : h->ev_pending) put_events(h, t);
+  for (cudaEvent_t e : h->ev_free) cudaEventDestroy(e);
   if (h->stream) cudaStreamDestroy(h->stream);
   delete h;
 }
@@ -996,10 +1006,12 @@ int twmc_sync(twmc_handle* h, double* kernel_ms) {
   if (e != cudaSuccess) return cuda_fail(h, e, "cudaStreamSynchronize");
   double ms = h->carry_ms;  // step launches of twmc_run calls since the last twmc_sync
   h->carry_ms = 0.0;
-  for (auto& ev : h->ev_pending) {
-    float x = 0;
-    if (cudaEventElapsedTime(&x, ev.first, ev.second) == cudaSuccess) ms += x;
-    h->ev_free.push_back(ev);
+  for (const StepTime& t : h->ev_pending) {
+    float most = 0, x = 0;
+    for (cudaEvent_t end : t.ends)
+      if (cudaEventElapsedTime(&x, t.first, end) == cudaSuccess) most = std::max(most, x);
+    ms += most;
+    put_events(h, t);
   }
   h->ev_pending.clear();
   if (kernel_ms) *kernel_ms = ms;
@@ -1159,13 +1171,16 @@ int twmc_run(twmc_handle* h, const twmc_task_desc* tasks, size_t n, twmc_outputs
       }};
       // Progress counts steps that have run: their launches' end events, looked
       // at after each frame is queued and waited for in order at the end.
-      std::vector<std::pair<cudaEvent_t, double>> marks;
+      std::vector<std::pair<std::vector<cudaEvent_t>, double>> marks;
       size_t marks_seen = 0;
-      auto mark = [&] { marks.push_back({h->ev_pending.back().second, total_steps ? double(done_steps) / double(total_steps) : 1.0}); };
+      auto mark = [&] { marks.push_back({h->ev_pending.back().ends, total_steps ? double(done_steps) / double(total_steps) : 1.0}); };
       auto look = [&](bool wait) {
         for (; marks_seen < marks.size(); ++marks_seen) {
-          const cudaError_t e = wait ? cudaEventSynchronize(marks[marks_seen].first) : cudaEventQuery(marks[marks_seen].first);
-          if (e != cudaSuccess) { if (e == cudaErrorNotReady) cudaGetLastError(); break; }
+          for (cudaEvent_t end : marks[marks_seen].first) {
+            const cudaError_t e = wait ? cudaEventSynchronize(end) : cudaEventQuery(end);
+            if (e == cudaErrorNotReady) cudaGetLastError();
+            if (e != cudaSuccess) return;
+          }
           h->progress = marks[marks_seen].second;
         }
       };
@@ -1211,10 +1226,7 @@ int twmc_run(twmc_handle* h, const twmc_task_desc* tasks, size_t n, twmc_outputs
         }
         double* snap = h->d_snap.as<double>();
         const float* st = static_cast<const float*>(h->d_state.p);
-        auto ev = get_events(h);
-        h->ev_pending.push_back(ev);
-        TWMC_CUDA(h, cudaEventRecord(ev.first, h->stream));
-        TWMC_CUDA(h, cudaEventRecord(ev.second, h->stream));  // (recorded again below: both stand on every exit)
+        start_timing(h);
         TWMC_CUDA(h, cudaEventRecord(h->fork, h->stream));
         for (int c = 0; c < kFinalChunks; ++c) {
           const int64_t t0 = int64_t(bn) * c / kFinalChunks, t1 = int64_t(bn) * (c + 1) / kFinalChunks;
@@ -1236,7 +1248,6 @@ int twmc_run(twmc_handle* h, const twmc_task_desc* tasks, size_t n, twmc_outputs
                                        snap + size_t(t0) * row, row, size_t(t1 - t0), h->dl_stream));
         }
         frame_sent = fdst != nullptr;
-        TWMC_CUDA(h, cudaEventRecord(ev.second, h->stream));
         TWMC_CUDA(h, cudaEventRecord(h->snap_free, h->dl_stream));
         h->step_pos += uint32_t(nsteps);
         final_sent = true;

@@ -23,10 +23,12 @@ struct Stream {
   std::deque<std::function<void()>> q;
   long issued = 0, done = 0;
   bool running = false;
+  double clock = 0.0;  // ms
 };
 struct Event {
   Stream* s = nullptr;
   long at = 0;
+  double time = 0.0;
 };
 
 namespace {
@@ -38,6 +40,11 @@ std::map<char*, size_t>& pinned() { static std::map<char*, size_t> m; return m; 
 size_t pinned_now = 0, pinned_peak = 0, pinned_limit = ~size_t(0);
 long g_uploads = 0, g_changed = 0, g_lowered = 0, g_launches = 0, g_fail_at = -1;
 std::string g_fail_name, g_log;
+std::map<std::string, double>& costs() { static std::map<std::string, double> m; return m; }
+double cost(const std::string& name) {
+  for (auto& e : costs()) if (name.find(e.first) != std::string::npos) return e.second;
+  return 0.0;
+}
 cudaError_t g_last = cudaSuccess;
 void (*g_hook)(const char*) = nullptr;
 struct Call { dim3 g, b; size_t m; cudaStream_t s; };
@@ -79,6 +86,7 @@ void fake_pinned_limit(size_t n) { pinned_limit = n; pinned_peak = pinned_now; }
 void fake_pin(void* p, size_t n) { pinned()[static_cast<char*>(p)] = n; }  // as cudaHostRegister
 void fake_fail_launch(const char* name, long nth) { g_fail_name = name; g_fail_at = nth; }  // the nth of that name from now on
 void fake_hook(void (*f)(const char*)) { g_hook = f; }  // called as each kernel runs
+void fake_cost(const char* name, double ms) { costs()[name] = ms; }  // of kernels by part of their name, and of "memcpy"
 const char* fake_log() { return g_log.c_str(); }
 
 // ---- registration and launches ----
@@ -105,7 +113,11 @@ cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3, dim3, void**, size_t m, cud
   if (g_fail_at >= 0 && name.find(g_fail_name) != std::string::npos && g_fail_at-- == 0) return ret(cudaErrorLaunchFailure);
   ++g_launches;
   g_log += name + "\n";
-  push(of(s), [name] { if (g_hook) g_hook(name.c_str()); });
+  Stream* st = of(s);
+  push(st, [name, st] {
+    st->clock += cost(name);
+    if (g_hook) g_hook(name.c_str());
+  });
   return cudaSuccess;
 }
 cudaError_t cudaFuncSetAttribute(const void* f, cudaFuncAttribute, int v) {
@@ -125,8 +137,10 @@ cudaError_t cudaEventCreate(cudaEvent_t* e) { return cudaEventCreateWithFlags(e,
 cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) {
   auto* p = reinterpret_cast<Event*>(e);
-  p->s = of(s);
-  p->at = of(s)->issued;
+  Stream* st = of(s);
+  push(st, [p, st] { p->time = st->clock; });
+  p->s = st;
+  p->at = st->issued;
   return cudaSuccess;
 }
 cudaError_t cudaEventSynchronize(cudaEvent_t e) { auto* p = reinterpret_cast<Event*>(e); if (p->s) drain(p->s, p->at); return cudaSuccess; }
@@ -134,10 +148,19 @@ cudaError_t cudaEventQuery(cudaEvent_t e) {
   auto* p = reinterpret_cast<Event*>(e);
   return !p->s || p->s->done >= p->at ? cudaSuccess : ret(cudaErrorNotReady);
 }
-cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t) { *ms = 1.0f; return cudaSuccess; }
+cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t a, cudaEvent_t b) {
+  *ms = float(reinterpret_cast<Event*>(b)->time - reinterpret_cast<Event*>(a)->time);
+  return cudaSuccess;
+}
 cudaError_t cudaStreamWaitEvent(cudaStream_t s, cudaEvent_t e, unsigned) {
-  const Event v = *reinterpret_cast<Event*>(e);
-  if (v.s && v.s != of(s)) push(of(s), [v] { drain(v.s, v.at); });
+  const auto* p = reinterpret_cast<Event*>(e);
+  const Event v = *p;
+  Stream* st = of(s);
+  if (v.s && v.s != st)
+    push(st, [v, p, st] {
+      drain(v.s, v.at);
+      if (p->at == v.at && p->time > st->clock) st->clock = p->time;  // (not recorded anew meanwhile)
+    });
   return cudaSuccess;
 }
 
@@ -175,13 +198,13 @@ cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind k, 
     });
     return cudaSuccess;
   }
-  push(of(st), [=] { std::memcpy(d, s, n); });
+  push(of(st), [=] { of(st)->clock += cost("memcpy"); std::memcpy(d, s, n); });
   if (k == cudaMemcpyDeviceToHost && !is_pinned(d)) drain(of(st), of(st)->issued);
   return cudaSuccess;
 }
 cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) { drain(&g_null, g_null.issued); std::memcpy(d, s, n); return cudaSuccess; }
 cudaError_t cudaMemcpy2DAsync(void* d, size_t dp, const void* s, size_t sp, size_t w, size_t h, cudaMemcpyKind k, cudaStream_t st) {
-  push(of(st), [=] { for (size_t i = 0; i < h; ++i) std::memcpy(static_cast<char*>(d) + i * dp, static_cast<const char*>(s) + i * sp, w); });
+  push(of(st), [=] { of(st)->clock += cost("memcpy"); for (size_t i = 0; i < h; ++i) std::memcpy(static_cast<char*>(d) + i * dp, static_cast<const char*>(s) + i * sp, w); });
   if (k == cudaMemcpyDeviceToHost && !is_pinned(d)) drain(of(st), of(st)->issued);
   return cudaSuccess;
 }

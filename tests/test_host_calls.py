@@ -21,6 +21,7 @@ lib.fake_pinned_peak.restype = C.c_size_t
 lib.fake_pinned_limit.argtypes = [C.c_size_t]
 lib.fake_fail_launch.argtypes = [C.c_char_p, C.c_long]
 lib.fake_log.restype = C.c_char_p
+lib.fake_cost.argtypes = [C.c_char_p, C.c_double]
 lib.fake_pin.argtypes = [C.c_void_p, C.c_size_t]
 def chain(n_traj, n_frames, sites=64):
     s = twmc.System(nx=1, ny=sites, J=1.0, dt=0.01, frame_steps=2, omega=-0.5, U=0.2, F=1.0, beta_init_sigma=0.5)
@@ -155,5 +156,28 @@ except twmc.TWMCError:
     pass
 lost = np.isnan(bufs["frames"]).any(axis=(0, 2))
 assert not lost[:4].any() and lost[4:].all(), lost
+s.close()
+""")
+
+
+@pytest.mark.parametrize("n_frames", [1, 3])
+def test_step_time_is_that_of_the_step_launches(script, n_frames):
+    """twmc_sync's step time after a run whose last steps go in ranges on streams
+    of their own, each followed by its widening and its copy home: the step
+    launches' time, overlapping ones counted once, and nothing else's."""
+    script(f"n_frames = {n_frames}" + """
+lib.fake_cost(b"fft_kernel", 1.0)
+lib.fake_cost(b"widen_kernel", 10.0)
+lib.fake_cost(b"memcpy", 100.0)
+s = twmc.System(nx=16, ny=16, J=1.0, dt=0.01, frame_steps=2, omega=-0.5, U=0.2, F=1.0, beta_init_sigma=0.5)
+t = s.make_tasks(4096, t_end=0.02 * n_frames, store_initial=False)
+for frames in (False, True):
+    s.run(t, frames=frames)
+    ms = s.sync()
+    assert n_frames <= ms <= n_frames + 3, ms   # each stretch once; the four ranges one after the other at most
+s.batch_init(t)
+s.advance(2); s.advance(2); s.reduce()
+assert s.sync() == 2.0
+assert s.sync() == 0.0
 s.close()
 """)
