@@ -174,6 +174,7 @@ def measure_batch(twmc, torch, sm_mhz=None, t_end=60.0):
     frames = int(round(t_end / (DT * FRAME_STEPS)))
     hb = twmc.HBatch(pts, FRAME_STEPS, tune=True)
     plans = [hb.plan(i) for i in range(len(pts))]
+    kernels = [hb.step_kernel(i) for i in range(len(pts))]
     hb.run(1)  # untimed first frame
     hb.sync()
     hb.run(frames)
@@ -186,7 +187,7 @@ def measure_batch(twmc, torch, sm_mhz=None, t_end=60.0):
     out = {"value": rate, "unit": METRIC, "points": len(pts), "t_end": t_end, "frames": frames,
            "device_s": ms / 1e3, "trajectories_per_s": sum(p["n_traj"] for p in pts) / (ms / 1e3),
            "finite": finite, "autotuned": True,
-           "kernels": dict(Counter(p.split("<")[0] for p in plans)),
+           "kernels": dict(sorted(Counter(kernels).items())),
            "variants": dict(sorted(Counter(p.split("<")[1].rstrip(">") for p in plans).items())),
            "timing": "CUDA events around the graph replays of frames 2..121 (t = 0.5..60.5, the 30000 steps of "
                      "a run to t_end = 60); trajectories_per_s = all points' trajectories / that time"}
@@ -209,7 +210,7 @@ def measure_other_paths(twmc, torch, sm_mhz=None):
     sysd = make_system(twmc, hop=twmc.HOP_STENCIL)
     s = workloads.time_batch(sysd, NTRAJ, 2)
     r = FRAME_STEPS * NTRAJ * NX * NY * 2 / s
-    out["headline_real_space"] = {"value": r, "unit": METRIC, "kernel": sysd.kernel_name, "ms_per_frame": s * 500}
+    out["headline_real_space"] = {"value": r, "unit": METRIC, "kernel": sysd.step_kernel, "ms_per_frame": s * 500}
     out["headline_real_space"]["issue"] = issue_fraction(r, "pair_kernel_64x64.md", sm_mhz, torch)
     sysd.close()
     out["heterogeneous_batch"] = measure_batch(twmc, torch, sm_mhz)
@@ -222,7 +223,7 @@ def measure_other_paths(twmc, torch, sm_mhz=None):
     el = time.perf_counter() - t0
     kms = sysd.sync()  # CUDA-event time of the step launches of the timed call
     r = sysd.n_sites * 8192 * 1000 / (kms / 1e3)
-    out["lieb"] = {"value": r, "unit": METRIC, "kernel": sysd.kernel_name, "kernel_ms_per_1000_steps": kms,
+    out["lieb"] = {"value": r, "unit": METRIC, "kernel": sysd.step_kernel, "kernel_ms_per_1000_steps": kms,
                    "workload": "1-D Lieb 256 cells x 3, PBC, U = 0.27 + 0.06 U[0,1), F(t) ramp on B sites, "
                                "8192 trajectories, 1000 steps (CUDA events around the step launches)",
                    "issue": issue_fraction(r, "lieb_pair_kernel_lieb768.md", sm_mhz, torch),
@@ -233,7 +234,7 @@ def measure_other_paths(twmc, torch, sm_mhz=None):
     sysd = workloads.square(128, 128, hop=twmc.HOP_STENCIL)
     s = workloads.time_batch(sysd, 4096, 1)
     r = 128 * 128 * 4096 * FRAME_STEPS / s
-    out["square128"] = {"value": r, "unit": METRIC, "kernel": sysd.kernel_name, "ms_per_frame": s * 1e3,
+    out["square128"] = {"value": r, "unit": METRIC, "kernel": sysd.step_kernel, "ms_per_frame": s * 1e3,
                         "workload": "128x128 PBC, the headline parameters, 4096 trajectories, one 250-step frame",
                         "issue": issue_fraction(r, "pair_cluster_kernel_128x128.md", sm_mhz, torch)}
     sysd.close()
@@ -257,7 +258,7 @@ def measure_f64(twmc, torch, steps=2, precision=None, integrator=0):
     e1.record(ext)
     sysd.sync()
     ms = e0.elapsed_time(e1)
-    kname = sysd.kernel_name
+    kname = sysd.step_kernel
     sysd.close()
     return {"value": steps * FRAME_STEPS * NTRAJ * NX * NY / (ms / 1e3), "unit": METRIC, "steps": steps,
             "kernel": kname}
@@ -534,7 +535,7 @@ def main():
                 "n_site_avg": float(np.mean(ens["n"])), "g2_site_avg": float(np.nanmean(ens["g2"])),
                 "merge": "moment blocks gathered in rank order (replicas.gather_blocks over gloo)" if dist else
                          "single rank"}
-    info_kernel = sysd.kernel_name
+    info_kernel = sysd.step_kernel
     sysd.close()
     su_rank = float(args.steps) * FRAME_STEPS * ntraj * NX * NY
     t_max = elapsed_ms

@@ -209,7 +209,7 @@ TWMC_API int twmc_batch_download(twmc_handle* h, double* field, double* moments)
 /* Kernel launches issued by this handle since creation (trajectory steps,
  * reductions, initialisation). */
 TWMC_API int64_t twmc_launch_count(const twmc_handle* h);
-/* Name of the step kernel variant the handle selected: "square_fft_kernel"
+/* Name of the step path the handle selected: "square_fft_kernel"
  * (register FFT; "square_fft_kernel<fast>" for its compiled-in common run:
  * FP32, Philox noise, scalar U and F; "square_fft_kernel<fast,split>" the same
  * with the split-step integrator), "ell_kernel<stencil>" / "ell_kernel<table>" (real space,
@@ -221,6 +221,12 @@ TWMC_API int64_t twmc_launch_count(const twmc_handle* h);
  * unpacked one) runs them. Kernels chosen at launch time are reported after
  * the first step. */
 TWMC_API const char* twmc_kernel_name(const twmc_handle* h);
+/* The step kernel of the handle's last launch, with its split ("" before the
+ * first): "pair_kernel<V,NB>" (packed pairs of sites, V rows by NB blocks a
+ * thread; "_wide", ",chain"), "pair_cluster_kernel<V,CTAs>" (packed, on a
+ * cluster), "lieb_pair_kernel" (packed pairs of Lieb cells), "ell_kernel
+ * <sites,threads>" and the names above where those kernels ran. */
+TWMC_API const char* twmc_step_kernel(const twmc_handle* h);
 /* The CUDA stream (cudaStream_t) all of the handle's work is issued on, for
  * callers that order their own work or record events against it. */
 TWMC_API void* twmc_stream(const twmc_handle* h);
@@ -299,8 +305,12 @@ TWMC_API int64_t twmc_hbatch_total_sites(const twmc_hbatch* b);
 TWMC_API int twmc_hbatch_block_means(twmc_hbatch* b, double* out);
 /* cudaStream_t the batch runs on. */
 TWMC_API void* twmc_hbatch_stream(const twmc_hbatch* b);
-/* Kernel the point runs on. */
+/* The point's plan: the family of its queue kernel, its step variant and its
+ * lattice. */
 TWMC_API const char* twmc_hbatch_plan(const twmc_hbatch* b, size_t point);
+/* The queue kernel that runs the point and its step body: "fft", "pair V,NB"
+ * or "pair V,CTAs" (packed), "ell", "ell_cluster", "ell_cluster_pow2". */
+TWMC_API const char* twmc_hbatch_step_kernel(const twmc_hbatch* b, size_t point);
 TWMC_API const char* twmc_hbatch_last_error(const twmc_hbatch* b);
 TWMC_API int64_t twmc_hbatch_launch_count(const twmc_hbatch* b);
 TWMC_API void twmc_hbatch_destroy(twmc_hbatch* b);

@@ -153,6 +153,7 @@ struct twmc_handle {
   double carry_ms = 0.0;  // step-kernel device time of the last twmc_run, not yet reported
   double progress = 0.0;
   LaunchInfo last_info;
+  std::string step_kernel;  // of the last launch
 };
 
 namespace {
@@ -540,6 +541,7 @@ int advance(twmc_handle* h, int64_t n, bool want_nk, int64_t t0 = 0, int64_t t1 
   if (!range_stream) start_timing(h);
   std::string err;
   bool ok;
+  h->last_info = LaunchInfo();
   if (h->use_fft) {
     ok = h->prec == 0 ? square_launch_f32(h->bx, h->by, a, nparams, stream, &h->last_info, &err)
                       : square_launch_f64(h->bx, h->by, a, nparams, stream, &h->last_info, &err);
@@ -553,6 +555,7 @@ int advance(twmc_handle* h, int64_t n, bool want_nk, int64_t t0 = 0, int64_t t1 
   h->ev_pending.back().ends.push_back(get_event(h));
   cudaEventRecord(h->ev_pending.back().ends.back(), stream);
   if (!ok) return fail(h, TWMC_ERR_CUDA, err);
+  h->step_kernel = h->last_info.kernel.empty() ? h->last_info.name : h->last_info.kernel;
   ++h->launches;
   if (!range_stream) h->step_pos += uint32_t(n);
   return TWMC_OK;
@@ -1036,6 +1039,8 @@ int twmc_batch_download(twmc_handle* h, double* field, double* moments) {
 int64_t twmc_launch_count(const twmc_handle* h) { return h ? h->launches : -1; }
 
 const char* twmc_kernel_name(const twmc_handle* h) { return h ? h->kname.c_str() : ""; }
+
+const char* twmc_step_kernel(const twmc_handle* h) { return h ? h->step_kernel.c_str() : ""; }
 
 void* twmc_stream(const twmc_handle* h) { return h ? reinterpret_cast<void*>(h->stream) : nullptr; }
 

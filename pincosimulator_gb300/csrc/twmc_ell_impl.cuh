@@ -40,7 +40,7 @@ bool ell_launch_t(const StepArgs& a0, cudaStream_t s, LaunchInfo* info, std::str
   if (e != cudaSuccess || per_sm <= 0) { cudaGetLastError(); if (err) *err = "ell kernel does not fit on an SM"; return false; }
   const int64_t groups = (a.ntraj + tpc - 1) / tpc;
   const int grid = int(std::min<int64_t>(groups, int64_t(sms) * per_sm));
-  if (info) { info->name = "ell_kernel"; info->cta = CTA; info->grid = grid; info->smem = smem; info->blocks_per_sm = per_sm; }
+  if (info) { info->name = "ell_kernel"; info->kernel = "ell_kernel<" + std::to_string(VPT) + "," + std::to_string(CTA) + ">"; info->cta = CTA; info->grid = grid; info->smem = smem; info->blocks_per_sm = per_sm; }
   if (grid <= 0) return true;
   fn<<<grid, CTA, smem, s>>>(a);
   e = cudaGetLastError();

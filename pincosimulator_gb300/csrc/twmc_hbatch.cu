@@ -124,6 +124,9 @@ struct PairSplit {
   int64_t rows = 0, ny = 0;  // of one CTA
   int code() const { return v == 0 ? 0 : (chain ? 4096 : 0) + cl * 256 + v * 16 + nb; }
   int tpt() const { return int((rows / v * ny + nb - 1) / nb); }
+  std::string name() const {
+    return "pair " + std::to_string(v) + "," + std::to_string(cl > 1 ? cl : nb) + (chain ? ",chain" : "");
+  }
 };
 #define TWMC_HB_CODE(V, NB, CH, CL) ((CH ? 4096 : 0) + CL * 256 + V * 16 + NB)
 // Splits of the 256- and 512-thread queues, preferred first for their slots
@@ -476,6 +479,7 @@ struct twmc_hbatch {
   std::vector<int> shape;          // register-FFT plan id per point (kVarFft), else its PairSplit code
   std::vector<PairSplit> split;    // of the real-space points
   std::vector<std::string> plan;
+  std::vector<std::string> kernel;  // queue kernel and step body of each point
   std::vector<int64_t> nsites, ntraj, off_state, nblocks;
   DBuf<float2> state;
   DBuf<float> nk;
@@ -744,6 +748,7 @@ int hb_build(twmc_hbatch* b, const twmc_point_desc* points, size_t n, int64_t fr
   b->shape.assign(n, 0);
   b->split.assign(n, PairSplit());
   b->plan.assign(n, "");
+  b->kernel.assign(n, "");
   std::map<std::string, std::string> cache;
   const std::string cpath = tune_cache_path();
   if (tune) cache = read_cache(cpath);
@@ -779,6 +784,10 @@ int hb_build(twmc_hbatch* b, const twmc_point_desc* points, size_t n, int64_t fr
     static const char* qname[kQueues] = {"hbatch_kernel", "hbatch_kernel_512", "hbatch_cluster_kernel", "hbatch_cluster_kernel"};
     b->plan[i] = std::string(qname[kVarQueue[v]]) + "<" + kVarName[v] + " " + std::to_string(d.nx) + "x" +
                  std::to_string(d.ny) + ">";
+    static const char* kname[kQueues] = {"hbatch_kernel", "hbatch_kernel_512", "hbatch_cluster_kernel", "hbatch_cluster4_kernel"};
+    const PairSplit& sp = b->split[i];
+    const char* body = v == kVarFft ? "fft" : v == kVarCluster ? "ell_cluster" : v == kVarClusterPow2 ? "ell_cluster_pow2" : "ell";
+    b->kernel[i] = std::string(kname[var_queue(v, sp)]) + "<" + (sp.v ? sp.name() : body) + ">";
   }
   if (cache_dirty) write_cache(cpath, cache);
   cudaSetDevice(b->device);
@@ -1098,6 +1107,11 @@ void* twmc_hbatch_stream(const twmc_hbatch* b) { return b ? static_cast<void*>(b
 const char* twmc_hbatch_plan(const twmc_hbatch* b, size_t point) {
   if (!b || point >= b->npts) return "";
   return b->plan[point].c_str();
+}
+
+const char* twmc_hbatch_step_kernel(const twmc_hbatch* b, size_t point) {
+  if (!b || point >= b->npts || point >= b->kernel.size()) return "";
+  return b->kernel[point].c_str();
 }
 
 const char* twmc_hbatch_last_error(const twmc_hbatch* b) { return b ? b->err.c_str() : "null batch"; }

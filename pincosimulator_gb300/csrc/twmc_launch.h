@@ -20,7 +20,8 @@ struct PlanView {
 };
 
 struct LaunchInfo {
-  const char* name = "";
+  const char* name = "";  // what twmc_kernel_name says
+  std::string kernel;     // the kernel launched, with its split
   int cta = 0;
   int grid = 0;
   size_t smem = 0;

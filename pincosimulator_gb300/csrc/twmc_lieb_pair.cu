@@ -40,7 +40,7 @@ bool lieb_pair_launch(const StepArgs& a, cudaStream_t s, LaunchInfo* info, std::
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
   if (e != cudaSuccess) { cudaGetLastError(); if (err) *err = std::string("packed Lieb smem: ") + cudaGetErrorString(e); return false; }
   const int64_t groups = (a.ntraj + tpc - 1) / tpc;
-  if (info) { info->name = "lieb_cell_kernel"; info->cta = threads; info->grid = int(groups); info->smem = smem; info->blocks_per_sm = 1; }
+  if (info) { info->name = "lieb_cell_kernel"; info->kernel = "lieb_pair_kernel"; info->cta = threads; info->grid = int(groups); info->smem = smem; info->blocks_per_sm = 1; }
   if (groups <= 0) return true;
   if (groups > int64_t(0x7fffffff)) { if (err) *err = "packed Lieb kernel: too many trajectories"; return false; }
   fn<<<unsigned(groups), unsigned(threads), smem, s>>>(a);

@@ -84,7 +84,11 @@ bool pair_launch_par(const StepArgs& a, const PairPlan& p, cudaStream_t s, Launc
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(p.smem));
   if (e != cudaSuccess) { cudaGetLastError(); if (err) *err = std::string("packed real-space smem: ") + cudaGetErrorString(e); return false; }
   const int64_t groups = p.cl > 1 ? a.ntraj : (a.ntraj + p.tpc - 1) / p.tpc;
-  if (info) { info->cta = p.threads; info->grid = int(groups * p.cl); info->smem = p.smem; info->blocks_per_sm = 1; }
+  if (info) {
+    info->kernel = std::string(p.cl > 1 ? "pair_cluster_kernel" : "pair_kernel") + (p.wide ? "_wide<" : "<") +
+                   std::to_string(p.v) + "," + std::to_string(p.cl > 1 ? p.cl : p.nb) + (p.chain ? ",chain>" : ">");
+    info->cta = p.threads; info->grid = int(groups * p.cl); info->smem = p.smem; info->blocks_per_sm = 1;
+  }
   if (groups <= 0) return true;
   if (groups * p.cl > int64_t(0x7fffffff)) { if (err) *err = "packed real-space kernel: too many trajectories"; return false; }
   fn<<<unsigned(groups * p.cl), unsigned(p.threads), p.smem, s>>>(a);

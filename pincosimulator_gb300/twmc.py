@@ -29,10 +29,10 @@ DISORDER_NONE, DISORDER_GAUSSIAN, DISORDER_UNIFORM = 0, 1, 2
 EXPORTED = [
     "twmc_version", "twmc_create", "twmc_run", "twmc_set_noise_buffer", "twmc_progress", "twmc_last_error",
     "twmc_destroy", "twmc_batch_init", "twmc_batch_advance", "twmc_batch_reduce", "twmc_sync",
-    "twmc_batch_download", "twmc_launch_count", "twmc_kernel_name", "twmc_stream", "twmc_measure_fp32_peak",
+    "twmc_batch_download", "twmc_launch_count", "twmc_kernel_name", "twmc_step_kernel", "twmc_stream", "twmc_measure_fp32_peak",
     "twmc_kspace_moments_noalloc", "twmc_debug_philox", "twmc_debug_wiener",
     "twmc_hbatch_create", "twmc_hbatch_create_variants", "twmc_hbatch_run", "twmc_hbatch_sync", "twmc_hbatch_moments", "twmc_hbatch_state",
-    "twmc_hbatch_plan", "twmc_hbatch_last_error", "twmc_hbatch_launch_count", "twmc_hbatch_destroy",
+    "twmc_hbatch_plan", "twmc_hbatch_step_kernel", "twmc_hbatch_last_error", "twmc_hbatch_launch_count", "twmc_hbatch_destroy",
     "twmc_hbatch_set_init", "twmc_hbatch_field_moments", "twmc_hbatch_total_sites", "twmc_hbatch_stream",
     "twmc_hbatch_block_means",
     "twmc_mlp_create", "twmc_mlp_param_count", "twmc_mlp_set_params", "twmc_mlp_get_params", "twmc_mlp_get_grads",
@@ -132,6 +132,10 @@ def load(path: Optional[str] = None):
     lib.twmc_launch_count.restype = C.c_int64
     lib.twmc_kernel_name.argtypes = [C.c_void_p]
     lib.twmc_kernel_name.restype = C.c_char_p
+    lib.twmc_step_kernel.argtypes = [C.c_void_p]
+    lib.twmc_step_kernel.restype = C.c_char_p
+    lib.twmc_hbatch_step_kernel.argtypes = [C.c_void_p, C.c_size_t]
+    lib.twmc_hbatch_step_kernel.restype = C.c_char_p
     lib.twmc_debug_philox.argtypes = [C.c_void_p, C.c_size_t, C.c_void_p, C.c_void_p]
     lib.twmc_debug_wiener.argtypes = [C.c_int32, C.c_uint32, C.c_uint64, C.c_uint32, C.c_int64, C.c_int64,
                                       C.c_void_p]
@@ -282,6 +286,11 @@ class System:
     @property
     def kernel_name(self) -> str:
         return self.lib.twmc_kernel_name(self.h).decode()
+
+    @property
+    def step_kernel(self) -> str:
+        """Step kernel of the last launch, with its split."""
+        return self.lib.twmc_step_kernel(self.h).decode()
 
     @property
     def stream(self) -> int:
@@ -465,6 +474,10 @@ class HBatch:
 
     def plan(self, i) -> str:
         return self.lib.twmc_hbatch_plan(self.h, i).decode()
+
+    def step_kernel(self, i) -> str:
+        """Queue kernel and step body that run point i."""
+        return self.lib.twmc_hbatch_step_kernel(self.h, i).decode()
 
     @property
     def stream(self) -> int:

@@ -143,7 +143,7 @@ def main(argv=None):
         sysd = square(L, L, hop=twmc.HOP_STENCIL if args.hop == "stencil" else twmc.HOP_FFT,
                       integrator=twmc.INTEGRATOR_SPLIT if args.integrator == "split" else twmc.INTEGRATOR_EULER)
         el, finite = time_batch(sysd, args.ntraj, args.frames), True
-    line = {"workload": args.workload, "ntraj": args.ntraj, "frames": args.frames, "kernel": sysd.kernel_name,
+    line = {"workload": args.workload, "ntraj": args.ntraj, "frames": args.frames, "kernel": sysd.step_kernel,
             "seconds": el, "site_updates_per_s": sysd.n_sites * args.ntraj * args.frames * sysd.desc.frame_steps / el,
             "finite": finite}
     sysd.close()

@@ -181,3 +181,49 @@ assert s.sync() == 2.0
 assert s.sync() == 0.0
 s.close()
 """)
+
+
+def test_step_kernel_names_the_kernel_launched(script):
+    script("""
+def last_step():
+    names = [n for n in lib.fake_log().decode().split() if "kernel" in n]
+    return [n for n in names if any(k in n for k in ("pair", "ell_", "lieb_cell", "fft_kernel"))][-1]
+def check(want, **kw):
+    a = dict(J=1.0, dt=0.01, frame_steps=2, omega=-0.5, U=0.2, F=1.0, hop=twmc.HOP_STENCIL)
+    a.update(kw)
+    s = twmc.System(**a)
+    assert s.step_kernel == ""
+    s.batch_init(s.make_tasks(7))
+    s.advance(1)
+    got = s.step_kernel
+    assert got.split("<")[0] in (want, want + "_wide"), (kw, got)
+    assert got.split("<")[0] + "I" in last_step(), (kw, got, last_step())
+    s.close()
+for nx, ny in [(1, 2), (2, 2), (6, 10), (50, 50), (64, 64), (1, 1000), (2, 2048)]:
+    for kw in ({}, dict(U=twmc.Noisy(0.2, 1, 0.1)), dict(omega=twmc.Noisy(0.2, 1, 0.1))):
+        check("pair_kernel", nx=nx, ny=ny, **kw)
+check("pair_kernel", nx=1, ny=8192)
+check("pair_cluster_kernel", nx=128, ny=128)
+check("pair_cluster_kernel", nx=80, ny=80)
+for nx, ny in [(5, 7), (7, 4), (25, 25), (49, 50)]:
+    check("ell_kernel", nx=nx, ny=ny)
+check("ell_kernel", nx=64, ny=64, precision=twmc.PREC_F64)
+check("ell_cluster_kernel", nx=99, ny=101)
+check("ell_cluster_pow2_kernel", nx=4, ny=4096)
+check("square_fft_kernel", nx=64, ny=64, hop=twmc.HOP_FFT)
+lieb = dict(lattice=twmc.LATTICE_LIEB, nx=1, J_AB=1.0, J_BC=1.0)
+check("lieb_pair_kernel", ny=8, **lieb)
+check("lieb_pair_kernel", ny=1024, **lieb)
+check("lieb_cell_kernel", ny=8, precision=twmc.PREC_F64, **lieb)
+check("ell_kernel", ny=7, **lieb)
+pts = lambda *shapes: [dict(nx=nx, ny=ny, dt=0.01, n_traj=3) for nx, ny in shapes]
+hb = twmc.HBatch(pts((1, 32), (6, 10), (5, 7), (128, 128), (80, 80), (81, 81), (4, 4096), (45, 90)), 10)
+kernels = [hb.step_kernel(i).split(" ")[0].rstrip(">") for i in range(8)]
+assert kernels == ["hbatch_kernel<fft", "hbatch_kernel<pair", "hbatch_kernel<ell", "hbatch_cluster4_kernel<pair",
+                   "hbatch_cluster_kernel<pair", "hbatch_cluster_kernel<ell_cluster",
+                   "hbatch_cluster_kernel<ell_cluster_pow2", "hbatch_kernel_512<ell"], kernels
+hb.close()
+hb = twmc.HBatch(pts((64, 64)), 10, variants=["rowrun"])
+assert hb.step_kernel(0) == "hbatch_kernel_512<pair 2,2>", hb.step_kernel(0)
+hb.close()
+""")
