@@ -271,7 +271,7 @@ typedef struct twmc_hbatch twmc_hbatch;
  * 4096-site lattices, the fullest real-space stencil, or the cluster form);
  * 1 = per shape, time every variant the shape admits once on a trial batch
  * and keep the fastest (cached in $TWMC_TUNE_CACHE or
- * ~/.cache/twmc_tune.json). */
+ * ~/.cache/twmc_tune.json, for the kernels of this build). */
 TWMC_API int twmc_hbatch_create(const twmc_point_desc* points, size_t n, int64_t frame_steps, int32_t tune,
                                 twmc_hbatch** out);
 /* The same with the step variant of every point given by name (variants[i],

@@ -51,9 +51,24 @@ def _deps_hash() -> str:
     return h.hexdigest()
 
 
+# what the heterogeneous batch's queue kernels are compiled from
+QUEUE_SOURCES = ["twmc_hbatch.cu", "twmc_pair.cuh", "twmc_square.cuh", "twmc_kernels.cuh", "twmc_common.cuh",
+                 "fft_plans.inc"]
+
+
+def queue_revision() -> str:
+    h = hashlib.sha256()
+    for name in QUEUE_SOURCES:
+        with open(os.path.join(CSRC, name), "rb") as f:
+            h.update(f.read())
+    return h.hexdigest()[:12]
+
+
 def _compile(src: str, verbose: bool) -> str:
     obj = os.path.join(BUILD, src.replace(".cu", ".o"))
     cmd = [NVCC, *ARCH, *FLAGS, "-c", os.path.join(CSRC, src), "-o", obj]
+    if src == "twmc_hbatch.cu":
+        cmd.append(f'-DTWMC_QUEUE_REVISION="{queue_revision()}"')
     if verbose:
         cmd.insert(1, "-Xptxas=-v")
     r = subprocess.run(cmd, capture_output=True, text=True)

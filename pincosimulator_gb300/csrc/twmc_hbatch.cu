@@ -21,8 +21,8 @@
 // variant the shape admits (FFT plan, real-space stencil with 2 / 4 / 8
 // sites per thread -- i.e. trajectories per CTA --, cluster forms)
 // on a trial batch of that point alone and keeps the fastest; choices are
-// cached per device and shape in a JSON file ($TWMC_TUNE_CACHE, default
-// ~/.cache/twmc_tune.json).
+// cached per device, revision of the queue kernels and shape in a JSON file
+// ($TWMC_TUNE_CACHE, default ~/.cache/twmc_tune.json).
 #include <algorithm>
 #include <cmath>
 #include <complex>
@@ -428,7 +428,13 @@ std::string tune_cache_path() {
   return std::string(home ? home : ".") + "/.cache/twmc_tune.json";
 }
 
-// cache: one line per entry: "<device>|<nx>x<ny>": "<variant name>"
+// Digest of the sources of the queue kernels: a choice holds for the kernels
+// that it was timed on.
+#ifndef TWMC_QUEUE_REVISION
+#error "TWMC_QUEUE_REVISION: set by the build (build_ext.py)"
+#endif
+
+// cache: one line per entry: "<device>|<revision>|<nx>x<ny>": "<variant name>"
 std::map<std::string, std::string> read_cache(const std::string& path) {
   std::map<std::string, std::string> m;
   std::ifstream f(path);
@@ -757,7 +763,7 @@ int hb_build(twmc_hbatch* b, const twmc_point_desc* points, size_t n, int64_t fr
     const twmc_point_desc& d = points[i];
     int v = forced ? forced[i] : default_var(d);
     if (!forced && tune) {
-      const std::string key = devname + "|" + std::to_string(d.nx) + "x" + std::to_string(d.ny);
+      const std::string key = devname + "|" TWMC_QUEUE_REVISION "|" + std::to_string(d.nx) + "x" + std::to_string(d.ny);
       std::lock_guard<std::mutex> lock(g_tune_mu);
       auto it = cache.find(key);
       int cached = -1;

@@ -227,3 +227,29 @@ hb = twmc.HBatch(pts((64, 64)), 10, variants=["rowrun"])
 assert hb.step_kernel(0) == "hbatch_kernel_512<pair 2,2>", hb.step_kernel(0)
 hb.close()
 """)
+
+
+def test_tuned_choices_hold_for_the_kernels_they_were_timed_on(script, tmp_path):
+    """A cached choice without the revision of the queue kernels is not taken, and
+    a new one is kept beside it. (The stand-in times nothing: the first variant
+    that a lattice admits wins.)"""
+    cache = tmp_path / "tune.json"
+    cache.write_text('{\n  "fake|64x64": "ell8w",\n  "fake|0123456789ab|64x64": "rowrun"\n}\n')
+    script(f"cache = {str(cache)!r}" + """
+import json, os
+os.environ["TWMC_TUNE_CACHE"] = cache
+from pincosimulator_gb300 import build_ext
+pts = [dict(nx=64, ny=64, dt=0.01, n_traj=3)]
+hb = twmc.HBatch(pts, 10, tune=True)
+assert "<fft " in hb.plan(0), hb.plan(0)
+hb.close()
+entries = json.load(open(cache))
+assert entries == {"fake|64x64": "ell8w", "fake|0123456789ab|64x64": "rowrun",
+                   "fake|" + build_ext.queue_revision() + "|64x64": "fft"}, entries
+text = open(cache).read().replace('"fft"', '"ell8w"')
+open(cache, "w").write(text)
+hb = twmc.HBatch(pts, 10, tune=True)
+assert "<ell8w " in hb.plan(0), hb.plan(0)
+assert open(cache).read() == text
+hb.close()
+""")
