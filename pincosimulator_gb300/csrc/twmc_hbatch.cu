@@ -32,8 +32,10 @@
 #include <fstream>
 #include <map>
 #include <mutex>
+#include <set>
 #include <sstream>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include <sys/stat.h>
@@ -773,8 +775,12 @@ int hb_build(twmc_hbatch* b, const twmc_point_desc* points, size_t n, int64_t fr
         v = cached;
       } else {
         double best = -1.0;
+        std::set<std::tuple<int, int, int>> timed;  // what runs under a name: queue, split, unpacked body
         for (int k = 0; k < kVarCount; ++k) {
           if (!var_ok(k, d)) continue;
+          const PairSplit sp = var_split(k, d);
+          const int body = sp.v ? -1 : k == kVarRowrun ? int(kVarEll8w) : k;
+          if (!timed.insert({var_queue(k, sp), sp.code(), body}).second) continue;  // the first name of the same
           const double r = trial_rate(d, k);
           if (r > best) { best = r; v = k; }
         }

@@ -253,3 +253,23 @@ assert "<ell8w " in hb.plan(0), hb.plan(0)
 assert open(cache).read() == text
 hb.close()
 """)
+
+
+@pytest.mark.parametrize("nx,ny,trials", [
+    (64, 64, 2),    # fft; rowrun and ell8w run the same split
+    (32, 32, 4),    # fft, ell4, ell8 (one split), rowrun and ell8w (another)
+    (128, 128, 1),  # both cluster names run clusters of four
+    (4, 4096, 2),   # no packed split: the two unpacked cluster bodies
+    (25, 25, 3),    # odd: ell4, ell8, ell8w
+])
+def test_tuner_times_each_kernel_once(script, tmp_path, nx, ny, trials):
+    """Variant names that run the same kernel on a lattice are one trial, and its
+    first name is kept, not the one that noise favours."""
+    script(f"nx, ny, trials, cache = {nx}, {ny}, {trials}, {str(tmp_path / 'c.json')!r}" + """
+import os
+os.environ["TWMC_TUNE_CACHE"] = cache
+hb = twmc.HBatch([dict(nx=nx, ny=ny, dt=0.01, n_traj=3)], 10, tune=True)
+queues = [n for n in lib.fake_log().decode().split() if "hbatch_kernel" in n or "hbatch_cluster" in n]
+assert len(queues) == trials + 1, queues   # and the batch itself
+hb.close()
+""")
