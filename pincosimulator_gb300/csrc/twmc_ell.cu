@@ -61,7 +61,7 @@ bool lieb_cell_launch(const StepArgs& a0, cudaStream_t s, LaunchInfo* info, std:
   int dev = 0, sms = 0, per_sm = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  cudaError_t e = allow_smem(fn);
   if (e != cudaSuccess) { cudaGetLastError(); if (err) *err = std::string("lieb smem: ") + cudaGetErrorString(e); return false; }
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kLiebCta, smem);
   if (e != cudaSuccess || per_sm <= 0) { cudaGetLastError(); if (err) *err = "lieb kernel does not fit on an SM"; return false; }
@@ -91,7 +91,7 @@ bool cluster_config(const void* fn, int64_t ntraj, int64_t nsites, size_t static
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   if (smem + static_smem > size_t(maxsm)) { if (err) *err = "ell cluster kernel: field does not fit"; return false; }
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  cudaError_t e = allow_smem(fn);
   if (e != cudaSuccess) { cudaGetLastError(); if (err) *err = std::string("ell cluster smem: ") + cudaGetErrorString(e); return false; }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2, 1, 1);

@@ -33,7 +33,7 @@ bool ell_launch_t(const StepArgs& a0, cudaStream_t s, LaunchInfo* info, std::str
   size_t smem = ell_state_bytes(true, tpc, a.nsites, sizeof(T)) + wbytes;
   if (smem > size_t(maxsm)) { a.dbuf = 0; smem = ell_state_bytes(false, tpc, a.nsites, sizeof(T)) + wbytes; }
   if (smem > size_t(maxsm)) { if (err) *err = "ell kernel: trajectory does not fit in shared memory"; return false; }
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  cudaError_t e = allow_smem(fn);
   if (e != cudaSuccess) { cudaGetLastError(); if (err) *err = std::string("ell smem: ") + cudaGetErrorString(e); return false; }
   int per_sm = 0;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, CTA, smem);

@@ -945,7 +945,7 @@ int hb_build(twmc_hbatch* b, const twmc_point_desc* points, size_t n, int64_t fr
     if (b->qn[q] == 0) continue;
     const size_t smem = b->qsmem[q];
     if (smem + sizeof(StepArgs) + 64 > size_t(maxsm)) return hfail(b, TWMC_ERR_INVALID, "batch queue: field does not fit");
-    cudaError_t e = cudaFuncSetAttribute(qfn[q], cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    cudaError_t e = allow_smem(qfn[q], sizeof(StepArgs) + 64);
     if (e != cudaSuccess) { cudaGetLastError(); return hfail(b, TWMC_ERR_CUDA, std::string("batch queue smem: ") + cudaGetErrorString(e)); }
     int slots = 0;
     if (q == kQCluster || q == kQCluster4) {

@@ -19,6 +19,18 @@ struct PlanView {
   int thr_last[32] = {0};
 };
 
+// Lets launches of fn use any dynamic shared memory that the device has beside
+// `fixed` bytes of its own. The limit belongs to the function, process-wide: set to
+// one launch's size it could be lowered by another thread between this one's
+// setting and its launch, which is then refused.
+template <class F>
+cudaError_t allow_smem(F fn, size_t fixed = 0) {
+  int dev = 0, most = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most - int(fixed));
+}
+
 struct LaunchInfo {
   const char* name = "";  // what twmc_kernel_name says
   std::string kernel;     // the kernel launched, with its split

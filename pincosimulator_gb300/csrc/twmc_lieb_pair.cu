@@ -37,7 +37,7 @@ bool lieb_pair_launch(const StepArgs& a, cudaStream_t s, LaunchInfo* info, std::
   const int want = int(std::max<int64_t>(1, std::min<int64_t>(128 / tpt, batch / (2 * sms))));
   const int threads = (tpt * want + 31) / 32 * 32, tpc = threads / tpt;
   const size_t smem = 2 * lieb_buffer_bytes(a.nsites / 3) * size_t(tpc);
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  cudaError_t e = allow_smem(fn);
   if (e != cudaSuccess) { cudaGetLastError(); if (err) *err = std::string("packed Lieb smem: ") + cudaGetErrorString(e); return false; }
   const int64_t groups = (a.ntraj + tpc - 1) / tpc;
   if (info) { info->name = "lieb_cell_kernel"; info->kernel = "lieb_pair_kernel"; info->cta = threads; info->grid = int(groups); info->smem = smem; info->blocks_per_sm = 1; }

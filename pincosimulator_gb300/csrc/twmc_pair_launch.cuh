@@ -81,7 +81,7 @@ bool pair_launch_par(const StepArgs& a, const PairPlan& p, cudaStream_t s, Launc
 #undef TWMC_X
 #undef TWMC_Y
   if (!fn) { if (err) *err = "packed real-space kernel: variant not compiled"; return false; }
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(p.smem));
+  cudaError_t e = allow_smem(fn);
   if (e != cudaSuccess) { cudaGetLastError(); if (err) *err = std::string("packed real-space smem: ") + cudaGetErrorString(e); return false; }
   const int64_t groups = p.cl > 1 ? a.ntraj : (a.ntraj + p.tpc - 1) / p.tpc;
   if (info) {

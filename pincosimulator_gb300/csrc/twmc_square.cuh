@@ -41,7 +41,7 @@ bool square_launch_t(const StepArgs& a, int nparams, cudaStream_t s, LaunchInfo*
     return false;
   }
   auto fn = square_fft_kernel<R, P, CTA, FAST, SPLIT>;
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  cudaError_t e = allow_smem(fn);
   if (e != cudaSuccess) {
     cudaGetLastError();
     if (err) *err = std::string("square kernel smem attribute: ") + cudaGetErrorString(e);

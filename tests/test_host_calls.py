@@ -273,3 +273,31 @@ queues = [n for n in lib.fake_log().decode().split() if "hbatch_kernel" in n or 
 assert len(queues) == trials + 1, queues   # and the batch itself
 hb.close()
 """)
+
+
+def test_shared_memory_limits_are_not_lowered(script):
+    """The limit of a kernel's dynamic shared memory is process-wide: a launch that
+    needs less must not lower it under another thread's launch that needs more."""
+    script("""
+def go(n_traj, **kw):
+    a = dict(J=1.0, dt=0.01, frame_steps=2, omega=-0.5, U=0.2, F=1.0, hop=twmc.HOP_STENCIL)
+    a.update(kw)
+    s = twmc.System(**a)
+    s.batch_init(s.make_tasks(n_traj))
+    s.advance(1)
+    s.close()
+for n_traj in (4000, 1, 300):
+    for nx, ny in [(32, 32), (16, 16), (64, 64), (50, 50), (6, 10), (128, 128), (80, 80), (96, 96), (99, 101), (5, 7),
+                   (4, 4096), (128, 4), (1, 4096), (1, 50)]:
+        go(n_traj, nx=nx, ny=ny)
+        go(n_traj, nx=nx, ny=ny, omega=twmc.Noisy(-0.5, 1, 0.2))
+    for cells in (256, 16, 7, 1024):
+        for prec in (twmc.PREC_F32, twmc.PREC_F64)[:1 if cells > 256 else 2]:  # 1024 cells fit in FP32 only
+            go(n_traj, lattice=twmc.LATTICE_LIEB, nx=1, ny=cells, J_AB=1.0, J_BC=1.0, precision=prec)
+    for integ in (twmc.INTEGRATOR_SPLIT, twmc.INTEGRATOR_EULER):
+        for prec in (twmc.PREC_F32, twmc.PREC_F64):
+            go(n_traj, nx=16, ny=16, hop=twmc.HOP_FFT, integrator=integ, precision=prec, U=twmc.Noisy(0.2, 1, 0.1))
+for shapes in ([(64, 64), (128, 128)], [(6, 10), (80, 80), (25, 25)], [(128, 128), (96, 96)], [(50, 50)], [(120, 100)]):
+    twmc.HBatch([dict(nx=nx, ny=ny, dt=0.01, n_traj=3) for nx, ny in shapes], 10).close()
+assert lib.fake_lowered() == 0, lib.fake_lowered()
+""")
