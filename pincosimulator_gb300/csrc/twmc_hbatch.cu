@@ -8,7 +8,8 @@
 // sites. Every (point, trajectory group) is a work item of a persistent
 // work-queue kernel -- one per CTA geometry: hbatch_kernel (256 threads),
 // hbatch_kernel_512, hbatch_cluster4_kernel (clusters of four 256-thread CTAs)
-// and hbatch_cluster_kernel (of two 1024-thread CTAs) -- whose CTAs take items from an atomic
+// and hbatch_cluster_kernel (of two 1024-thread CTAs), with kernels of their own
+// for the unpacked bodies of 512 and 1024 threads (..._ell) -- whose CTAs take items from an atomic
 // counter, longest item first, and run the variant's step body for that
 // point (arguments and tables reloaded into shared memory when the point
 // changes). One frame -- counter reset, the queues on parallel graph
@@ -101,22 +102,25 @@ __device__ __forceinline__ void hb_run(unsigned char* smem, const StepArgs& a, b
   g.run(a, group, buf);
 }
 
-// Step variants of a batch point. Each runs in one of four persistent
+// Step variants of a batch point. Each runs in one of the persistent
 // work-queue kernels, by CTA geometry: 256 threads (register-FFT plans and
 // real-space stencils with 2, 4 or 8 sites per thread), 512 threads (8 sites
 // per thread, "rowrun" and "ell8w") and, for lattices above 4096 sites,
 // clusters: 4 CTAs of 256 threads where the packed form splits that way, else
 // 2 CTAs of 1024 threads. Real-space points run the packed body
 // (twmc_pair.cuh) wherever their lattice pairs up and splits into their
-// variant's threads, else the unpacked bodies.
+// variant's threads, else the unpacked bodies. At 512 and 1024 threads these have
+// kernels of their own: beside the packed body's calls they lost 3 to 6 %
+// (GB300, ms per 250 steps of 500 trajectories, apart and together: 45x90
+// 2.23 / 2.30, 81x81 7.40 / 7.80); at 256 threads it is the same (25x25 0.63).
 enum HbVariant : int {
   kVarFft = 0, kVarEll2, kVarEll4, kVarEll8, kVarRowrun, kVarEll8w, kVarClusterPow2, kVarCluster, kVarCount
 };
 constexpr const char* kVarName[kVarCount] = {"fft", "ell2", "ell4", "ell8", "rowrun", "ell8w", "cluster_pow2",
                                              "cluster"};
-enum HbQueue : int { kQ256 = 0, kQ512, kQCluster, kQCluster4, kQueues };
+enum HbQueue : int { kQ256 = 0, kQ512, kQCluster, kQCluster4, kQ512Ell, kQClusterEll, kQueues };
 constexpr int kVarQueue[kVarCount] = {kQ256, kQ256, kQ256, kQ256, kQ512, kQ512, kQCluster, kQCluster};
-constexpr int kQueueCta[kQueues] = {256, 512, 1024, 256};
+constexpr int kQueueCta[kQueues] = {256, 512, 1024, 256, 512, 1024};
 
 // The packed body's split of a real-space point: V rows per block, NB blocks
 // per thread, chain or not, CTAs per trajectory; 0 = the unpacked body.
@@ -221,7 +225,8 @@ hbatch_kernel(const StepArgs* __restrict__ pts, const int* __restrict__ pvar, co
   }
 }
 
-// 512-thread queue: eight sites per thread.
+// 512-thread queues: eight sites per thread, packed, or unpacked through a
+// function (inlined into the item loop it ran 45x90 in 2.31 ms instead of 2.23).
 __global__ void __launch_bounds__(512, 1)
 hbatch_kernel_512(const StepArgs* __restrict__ pts, const int* __restrict__ pshape, const int2* __restrict__ items,
                   int nitems, int* __restrict__ counter) {
@@ -237,9 +242,22 @@ hbatch_kernel_512(const StepArgs* __restrict__ pts, const int* __restrict__ psha
   case TWMC_HB_CODE(V, NB, CH, 1): hb_pair<V, NB, CH>(s_a, smem_raw, w.y); break;
       TWMC_HB_SPLITS_512(TWMC_HB_CASE)
 #undef TWMC_HB_CASE
-      default: ell_body<float, 8, 512, 1, true>(s_a, smem_raw, w.y, kOneGroup); break;
+      default: break;
     }
   }
+}
+__device__ __noinline__ void hb_ell512(const StepArgs& a, unsigned char* smem_raw, int64_t group) {
+  ell_body<float, 8, 512, 1, true>(a, smem_raw, group, kOneGroup);
+}
+__global__ void __launch_bounds__(512, 1)
+hbatch_kernel_512_ell(const StepArgs* __restrict__ pts, const int2* __restrict__ items, int nitems, int* __restrict__ counter) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ __align__(16) StepArgs s_a;
+  __shared__ int s_item;
+  int cur = -1;
+  int2 w;
+  bool reload;
+  while (hb_next(pts, items, nitems, counter, s_a, s_item, cur, w, reload)) hb_ell512(s_a, smem_raw, w.y);
 }
 
 // Cluster queues: one item is one trajectory, run by all CTAs of a cluster;
@@ -273,8 +291,8 @@ __device__ __forceinline__ void hb_cluster_loop(const StepArgs* __restrict__ pts
 }
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(1024, 1)
-hbatch_cluster_kernel(const StepArgs* __restrict__ pts, const int* __restrict__ pvar, const int* __restrict__ pshape,
-                      const int2* __restrict__ items, int nitems, int* __restrict__ counter) {
+hbatch_cluster_kernel(const StepArgs* __restrict__ pts, const int* __restrict__ pshape, const int2* __restrict__ items,
+                      int nitems, int* __restrict__ counter) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(16) StepArgs s_a;
   __shared__ int s_item;
@@ -284,11 +302,41 @@ hbatch_cluster_kernel(const StepArgs* __restrict__ pts, const int* __restrict__ 
       case TWMC_HB_CODE(5, 1, false, 2): hb_pair<5, 1, false, 2>(s_a, smem_raw, w.y); break;
       case TWMC_HB_CODE(3, 1, false, 2): hb_pair<3, 1, false, 2>(s_a, smem_raw, w.y); break;
       case TWMC_HB_CODE(1, 1, false, 2): hb_pair<1, 1, false, 2>(s_a, smem_raw, w.y); break;
-      default:
-        if (pvar[w.x] == kVarClusterPow2) ell_cluster_pow2_body<1024, true>(s_a, smem_raw, w.y, kOneGroup);
-        else ell_cluster_body<float, 1024>(s_a, smem_raw, w.y, kOneGroup);
+      default: break;
     }
   });
+}
+
+// The unpacked bodies: the item loop written out (through hb_cluster_loop it
+// spilled 8 bytes more and ran 5 % slower).
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(1024, 1)
+hbatch_cluster_kernel_ell(const StepArgs* __restrict__ pts, const int* __restrict__ pvar, const int2* __restrict__ items,
+                          int nitems, int* __restrict__ counter) {
+  namespace cg = cooperative_groups;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ __align__(16) StepArgs s_a;
+  __shared__ int s_item;
+  cg::cluster_group cl = cg::this_cluster();
+  const unsigned rank = cl.block_rank();
+  int cur = -1;
+  for (;;) {
+    cl.sync();  // both ranks are done with the previous item (buffers, peer reads, s_item)
+    if (rank == 0 && threadIdx.x == 0) s_item = atomicAdd(counter, 1);
+    cl.sync();
+    const int it = rank == 0 ? s_item : *cl.map_shared_rank(&s_item, 0);
+    if (it >= nitems) break;
+    const int2 w = items[it];
+    if (w.x != cur) {
+      __syncthreads();
+      for (int i = threadIdx.x; i < int(sizeof(StepArgs) / 4); i += 1024)
+        reinterpret_cast<uint32_t*>(&s_a)[i] = reinterpret_cast<const uint32_t*>(pts + w.x)[i];
+      __syncthreads();
+      cur = w.x;
+    }
+    if (pvar[w.x] == kVarClusterPow2) ell_cluster_pow2_body<1024, true>(s_a, smem_raw, w.y, kOneGroup);
+    else ell_cluster_body<float, 1024>(s_a, smem_raw, w.y, kOneGroup);
+  }
+  cl.sync();  // rank 0's shared memory stays until rank 1 has read the last item index
 }
 
 // Clusters of four 256-thread CTAs, two CTAs per SM: while one waits at its
@@ -649,7 +697,11 @@ PairSplit var_split(int v, const twmc_point_desc& d) {
 }
 
 // Queue of a point.
-int var_queue(int v, const PairSplit& s) { return s.v && s.cl == 4 ? kQCluster4 : kVarQueue[v]; }
+int var_queue(int v, const PairSplit& s) {
+  const int q = kVarQueue[v];
+  if (s.v) return s.cl == 4 ? int(kQCluster4) : q;
+  return q == kQ512 ? int(kQ512Ell) : q == kQCluster ? int(kQClusterEll) : q;
+}
 
 // Threads per trajectory of the real-space variants, and trajectories per
 // work item of every variant.
@@ -793,10 +845,11 @@ int hb_build(twmc_hbatch* b, const twmc_point_desc* points, size_t n, int64_t fr
     b->var[i] = v;
     b->split[i] = var_split(v, d);
     b->shape[i] = v == kVarFft ? hb_shape_id(lg2(d.nx), lg2(d.ny)) : b->split[i].code();
-    static const char* qname[kQueues] = {"hbatch_kernel", "hbatch_kernel_512", "hbatch_cluster_kernel", "hbatch_cluster_kernel"};
+    static const char* qname[] = {"hbatch_kernel", "hbatch_kernel_512", "hbatch_cluster_kernel"};
     b->plan[i] = std::string(qname[kVarQueue[v]]) + "<" + kVarName[v] + " " + std::to_string(d.nx) + "x" +
                  std::to_string(d.ny) + ">";
-    static const char* kname[kQueues] = {"hbatch_kernel", "hbatch_kernel_512", "hbatch_cluster_kernel", "hbatch_cluster4_kernel"};
+    static const char* kname[kQueues] = {"hbatch_kernel", "hbatch_kernel_512", "hbatch_cluster_kernel",
+                                         "hbatch_cluster4_kernel", "hbatch_kernel_512_ell", "hbatch_cluster_kernel_ell"};
     const PairSplit& sp = b->split[i];
     const char* body = v == kVarFft ? "fft" : v == kVarCluster ? "ell_cluster" : v == kVarClusterPow2 ? "ell_cluster_pow2" : "ell";
     b->kernel[i] = std::string(kname[var_queue(v, sp)]) + "<" + (sp.v ? sp.name() : body) + ">";
@@ -940,7 +993,9 @@ int hb_build(twmc_hbatch* b, const twmc_point_desc* points, size_t n, int64_t fr
   const void* qfn[kQueues] = {reinterpret_cast<const void*>(hbatch_kernel),
                               reinterpret_cast<const void*>(hbatch_kernel_512),
                               reinterpret_cast<const void*>(hbatch_cluster_kernel),
-                              reinterpret_cast<const void*>(hbatch_cluster4_kernel)};
+                              reinterpret_cast<const void*>(hbatch_cluster4_kernel),
+                              reinterpret_cast<const void*>(hbatch_kernel_512_ell),
+                              reinterpret_cast<const void*>(hbatch_cluster_kernel_ell)};
   for (int q = 0; q < kQueues; ++q) {
     if (b->qn[q] == 0) continue;
     const size_t smem = b->qsmem[q];
@@ -948,8 +1003,8 @@ int hb_build(twmc_hbatch* b, const twmc_point_desc* points, size_t n, int64_t fr
     cudaError_t e = allow_smem(qfn[q], sizeof(StepArgs) + 64);
     if (e != cudaSuccess) { cudaGetLastError(); return hfail(b, TWMC_ERR_CUDA, std::string("batch queue smem: ") + cudaGetErrorString(e)); }
     int slots = 0;
-    if (q == kQCluster || q == kQCluster4) {
-      const int cl = q == kQCluster ? 2 : 4;
+    if (q == kQCluster || q == kQCluster4 || q == kQClusterEll) {
+      const int cl = q == kQCluster4 ? 4 : 2;
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3(cl, 1, 1);
       cfg.blockDim = dim3(kQueueCta[q], 1, 1);
@@ -982,10 +1037,16 @@ int hb_build(twmc_hbatch* b, const twmc_point_desc* points, size_t n, int64_t fr
         b->args.p, b->pshape.p, b->qitems[kQ512].p, b->qn[kQ512], b->counter.p + kQ512);
   if (b->qn[kQCluster] > 0)
     hbatch_cluster_kernel<<<b->qgrid[kQCluster], 1024, b->qsmem[kQCluster], b->sq[kQCluster]>>>(
-        b->args.p, b->pvar.p, b->pshape.p, b->qitems[kQCluster].p, b->qn[kQCluster], b->counter.p + kQCluster);
+        b->args.p, b->pshape.p, b->qitems[kQCluster].p, b->qn[kQCluster], b->counter.p + kQCluster);
   if (b->qn[kQCluster4] > 0)
     hbatch_cluster4_kernel<<<b->qgrid[kQCluster4], 256, b->qsmem[kQCluster4], b->sq[kQCluster4]>>>(
         b->args.p, b->qitems[kQCluster4].p, b->qn[kQCluster4], b->counter.p + kQCluster4);
+  if (b->qn[kQ512Ell] > 0)
+    hbatch_kernel_512_ell<<<b->qgrid[kQ512Ell], 512, b->qsmem[kQ512Ell], b->sq[kQ512Ell]>>>(
+        b->args.p, b->qitems[kQ512Ell].p, b->qn[kQ512Ell], b->counter.p + kQ512Ell);
+  if (b->qn[kQClusterEll] > 0)
+    hbatch_cluster_kernel_ell<<<b->qgrid[kQClusterEll], 1024, b->qsmem[kQClusterEll], b->sq[kQClusterEll]>>>(
+        b->args.p, b->pvar.p, b->qitems[kQClusterEll].p, b->qn[kQClusterEll], b->counter.p + kQClusterEll);
   cudaError_t le = cudaGetLastError();
   for (int q = 0; q < kQueues; ++q) {
     cudaEventRecord(b->qjoin[q], b->sq[q]);

@@ -220,8 +220,8 @@ pts = lambda *shapes: [dict(nx=nx, ny=ny, dt=0.01, n_traj=3) for nx, ny in shape
 hb = twmc.HBatch(pts((1, 32), (6, 10), (5, 7), (128, 128), (80, 80), (81, 81), (4, 4096), (45, 90)), 10)
 kernels = [hb.step_kernel(i).split(" ")[0].rstrip(">") for i in range(8)]
 assert kernels == ["hbatch_kernel<fft", "hbatch_kernel<pair", "hbatch_kernel<ell", "hbatch_cluster4_kernel<pair",
-                   "hbatch_cluster_kernel<pair", "hbatch_cluster_kernel<ell_cluster",
-                   "hbatch_cluster_kernel<ell_cluster_pow2", "hbatch_kernel_512<ell"], kernels
+                   "hbatch_cluster_kernel<pair", "hbatch_cluster_kernel_ell<ell_cluster",
+                   "hbatch_cluster_kernel_ell<ell_cluster_pow2", "hbatch_kernel_512_ell<ell"], kernels
 hb.close()
 hb = twmc.HBatch(pts((64, 64)), 10, variants=["rowrun"])
 assert hb.step_kernel(0) == "hbatch_kernel_512<pair 2,2>", hb.step_kernel(0)
