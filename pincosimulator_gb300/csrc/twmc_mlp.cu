@@ -292,8 +292,10 @@ __global__ void cast_params_kernel(const float* __restrict__ w, bf16* __restrict
 // 4); refreshes the BF16 copy. c1 = 1 / (1 - beta1^t), c2 = 1 / (1 - beta2^t).
 __device__ __forceinline__ float adam_one(float w, float g, float& m, float& v, float lr, float b1, float b2, float eps,
                                           float c1, float c2) {
-  m = b1 * m + (1.0f - b1) * g;
-  v = b2 * v + (1.0f - b2) * g * g;
+  // (one rounding for each form of the kernel: left to the compiler, the two
+  // contracted these sums differently)
+  m = __fmaf_rn(1.0f - b1, g, __fmul_rn(b1, m));
+  v = __fmaf_rn(__fmul_rn(1.0f - b2, g), g, __fmul_rn(b2, v));
   return w - lr * (m * c1) / (sqrtf(v * c2) + eps);
 }
 // Parameters from which P is 4. GB300, us per step with 1 and 4 per thread:

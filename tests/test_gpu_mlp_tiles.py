@@ -75,3 +75,31 @@ def test_a_row_does_not_depend_on_the_tile(built_lib):
     torch.cuda.synchronize()
     assert torch.equal(y[0, :128], y[1, :128])
     net.close()
+
+
+@pytest.mark.parametrize("widths", [[5, 64, 48, 37], [5, 256, 256, 256, 513], FULL])
+def test_adam_rounds_alike_for_every_size(built_lib, widths):
+    """One parameter per thread (small networks) or four: the same operations in
+    FP32, m = fma(1 - b1, g, b1 m) and v = fma((1 - b2) g, g, b2 v), bit for
+    bit over three steps."""
+    net, p, x, t = setup_net(widths, 64, 6)
+    xd, td = torch.as_tensor(x).cuda(), torch.as_tensor(t).cuda()
+    torch.cuda.synchronize()
+    f = np.float32
+    lr, b1, b2, eps, one = f(2e-3), f(0.9), f(0.999), f(1e-8), f(1)
+
+    def fma(a, b, c):
+        return (np.float64(a) * np.float64(b) + np.float64(c)).astype(f)  # the product is exact
+
+    w = p.astype(f)
+    m, v = np.zeros_like(w), np.zeros_like(w)
+    for step in range(1, 4):
+        net.backward(xd.data_ptr(), td.data_ptr(), 64)
+        g = net.get_grads()
+        net.adam(2e-3)
+        m = fma(one - b1, g, b1 * m)
+        v = fma((one - b2) * g, g, b2 * v)
+        c1, c2 = f(1 / (1 - float(b1) ** step)), f(1 / (1 - float(b2) ** step))
+        w = w - lr * (m * c1) / (np.sqrt(v * c2) + eps)
+        assert np.array_equal(net.get_params(), w), step
+    net.close()
