@@ -109,10 +109,13 @@ __device__ __forceinline__ void hb_run(unsigned char* smem, const StepArgs& a, b
 // clusters: 4 CTAs of 256 threads where the packed form splits that way, else
 // 2 CTAs of 1024 threads. Real-space points run the packed body
 // (twmc_pair.cuh) wherever their lattice pairs up and splits into their
-// variant's threads, else the unpacked bodies. At 512 and 1024 threads these have
-// kernels of their own: beside the packed body's calls they lost 3 to 6 %
-// (GB300, ms per 250 steps of 500 trajectories, apart and together: 45x90
-// 2.23 / 2.30, 81x81 7.40 / 7.80); at 256 threads it is the same (25x25 0.63).
+// variant's threads, else the unpacked bodies. On clusters these have a kernel of
+// their own: beside the packed body's calls they lost 5 % (GB300, ms per 250
+// steps of 500 trajectories: 81x81 7.40 apart, 7.80 together). At 512 threads a
+// batch whose points are all unpacked runs them so too (45x90 2.23 and 2.31); with
+// packed points they share a queue (and the packed functions' registers, which
+// ptxas allots by their callers: 64x64 ran 1.28 ms in this kernel, 1.36 in one
+// without the unpacked body). At 256 threads it is the same (25x25 0.63).
 enum HbVariant : int {
   kVarFft = 0, kVarEll2, kVarEll4, kVarEll8, kVarRowrun, kVarEll8w, kVarClusterPow2, kVarCluster, kVarCount
 };
@@ -225,8 +228,8 @@ hbatch_kernel(const StepArgs* __restrict__ pts, const int* __restrict__ pvar, co
   }
 }
 
-// 512-thread queues: eight sites per thread, packed, or unpacked through a
-// function (inlined into the item loop it ran 45x90 in 2.31 ms instead of 2.23).
+// 512-thread queues: eight sites per thread; all points, or unpacked ones alone,
+// through a function (inlined into the item loop: 45x90 2.31 ms instead of 2.23).
 __global__ void __launch_bounds__(512, 1)
 hbatch_kernel_512(const StepArgs* __restrict__ pts, const int* __restrict__ pshape, const int2* __restrict__ items,
                   int nitems, int* __restrict__ counter) {
@@ -242,7 +245,7 @@ hbatch_kernel_512(const StepArgs* __restrict__ pts, const int* __restrict__ psha
   case TWMC_HB_CODE(V, NB, CH, 1): hb_pair<V, NB, CH>(s_a, smem_raw, w.y); break;
       TWMC_HB_SPLITS_512(TWMC_HB_CASE)
 #undef TWMC_HB_CASE
-      default: break;
+      default: ell_body<float, 8, 512, 1, true>(s_a, smem_raw, w.y, kOneGroup); break;
     }
   }
 }
@@ -696,11 +699,11 @@ PairSplit var_split(int v, const twmc_point_desc& d) {
   return best;
 }
 
-// Queue of a point.
-int var_queue(int v, const PairSplit& s) {
+// Queue of a point; packed512: the batch has packed points of 512 threads.
+int var_queue(int v, const PairSplit& s, bool packed512) {
   const int q = kVarQueue[v];
   if (s.v) return s.cl == 4 ? int(kQCluster4) : q;
-  return q == kQ512 ? int(kQ512Ell) : q == kQCluster ? int(kQClusterEll) : q;
+  return q == kQ512 && !packed512 ? int(kQ512Ell) : q == kQCluster ? int(kQClusterEll) : q;
 }
 
 // Threads per trajectory of the real-space variants, and trajectories per
@@ -832,7 +835,7 @@ int hb_build(twmc_hbatch* b, const twmc_point_desc* points, size_t n, int64_t fr
           if (!var_ok(k, d)) continue;
           const PairSplit sp = var_split(k, d);
           const int body = sp.v ? -1 : k == kVarRowrun ? int(kVarEll8w) : k;
-          if (!timed.insert({var_queue(k, sp), sp.code(), body}).second) continue;  // the first name of the same
+          if (!timed.insert({var_queue(k, sp, false), sp.code(), body}).second) continue;  // the first name of the same
           const double r = trial_rate(d, k);
           if (r > best) { best = r; v = k; }
         }
@@ -848,13 +851,20 @@ int hb_build(twmc_hbatch* b, const twmc_point_desc* points, size_t n, int64_t fr
     static const char* qname[] = {"hbatch_kernel", "hbatch_kernel_512", "hbatch_cluster_kernel"};
     b->plan[i] = std::string(qname[kVarQueue[v]]) + "<" + kVarName[v] + " " + std::to_string(d.nx) + "x" +
                  std::to_string(d.ny) + ">";
+  }
+  if (cache_dirty) write_cache(cpath, cache);
+  bool packed512 = false;
+  for (size_t i = 0; i < n; ++i) packed512 |= kVarQueue[b->var[i]] == kQ512 && b->split[i].v != 0;
+  std::vector<int> queue(n);
+  for (size_t i = 0; i < n; ++i) {
     static const char* kname[kQueues] = {"hbatch_kernel", "hbatch_kernel_512", "hbatch_cluster_kernel",
                                          "hbatch_cluster4_kernel", "hbatch_kernel_512_ell", "hbatch_cluster_kernel_ell"};
     const PairSplit& sp = b->split[i];
+    const int v = b->var[i];
     const char* body = v == kVarFft ? "fft" : v == kVarCluster ? "ell_cluster" : v == kVarClusterPow2 ? "ell_cluster_pow2" : "ell";
-    b->kernel[i] = std::string(kname[var_queue(v, sp)]) + "<" + (sp.v ? sp.name() : body) + ">";
+    queue[i] = var_queue(v, sp, packed512);
+    b->kernel[i] = std::string(kname[queue[i]]) + "<" + (sp.v ? sp.name() : body) + ">";
   }
-  if (cache_dirty) write_cache(cpath, cache);
   cudaSetDevice(b->device);
 
   // layout and buffers
@@ -952,7 +962,7 @@ int hb_build(twmc_hbatch* b, const twmc_point_desc* points, size_t n, int64_t fr
     a.ktab = b->kt.p + tw_off[i];
     a.tpt = var_tpt(v, b->nsites[i], b->split[i]);
     a.dbuf = 1;
-    const int q = var_queue(v, b->split[i]);
+    const int q = queue[i];
     const int tpc = var_tpc(v, points[i], b->shape[i], b->split[i]);
     order[q].push_back({double(b->nsites[i]) * double(tpc), i});
     b->qsmem[q] = std::max(b->qsmem[q], var_smem(v, points[i], b->shape[i], b->split[i]));

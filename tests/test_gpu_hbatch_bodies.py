@@ -78,3 +78,19 @@ def test_unpacked_points_match_single_runs(built_lib, variant):
         e = np.abs(hb.state(i) - f).max() / np.abs(f).max()
         assert e < 1e-5, (p, hb.step_kernel(i), kernel, e)
     hb.close()
+
+
+def test_packed_and_unpacked_points_in_one_batch(built_lib):
+    """Every queue at once, and 512-thread points of both kinds in one."""
+    pts = points([(64, 64), (63, 64), (45, 90), (50, 50), (128, 128), (81, 81), (4, 4096), (80, 80), (5, 7), (6, 10)])
+    variants = ["ell8w", "ell8w", "ell8w", "ell8w", "cluster", "cluster", "cluster_pow2", "cluster", "ell2", "ell2"]
+    hb = twmc.HBatch(pts, FS, variants=variants)
+    hb.run(FRAMES)
+    hb.sync()
+    for i, p in enumerate(pts):
+        f, kernel = single(p)
+        packed = "<pair " in hb.step_kernel(i)
+        assert packed == kernel.startswith("pair_"), (p, hb.step_kernel(i), kernel)
+        e = np.abs(hb.state(i) - f).max() / np.abs(f).max()
+        assert e == 0 if packed else e < 1e-5, (p, hb.step_kernel(i), kernel, e)
+    hb.close()

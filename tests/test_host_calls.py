@@ -226,6 +226,9 @@ hb.close()
 hb = twmc.HBatch(pts((64, 64)), 10, variants=["rowrun"])
 assert hb.step_kernel(0) == "hbatch_kernel_512<pair 2,2>", hb.step_kernel(0)
 hb.close()
+hb = twmc.HBatch(pts((64, 64), (63, 64)), 10, variants=["ell8w", "ell8w"])   # one queue for both
+assert [hb.step_kernel(i) for i in range(2)] == ["hbatch_kernel_512<pair 2,2>", "hbatch_kernel_512<ell>"]
+hb.close()
 """)
 
 
