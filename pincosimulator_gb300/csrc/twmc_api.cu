@@ -1175,12 +1175,13 @@ int twmc_run(twmc_handle* h, const twmc_task_desc* tasks, size_t n, twmc_outputs
                           size_t(placed) * row * sizeof(double), bn, cudaMemcpyDeviceToHost, h->stream);
       }};
       // Progress counts steps that have run: their launches' end events, looked
-      // at after each frame is queued and waited for in order at the end.
+      // at after each frame is queued and waited for in order at the end (but the
+      // last, which the wait for the stream covers).
       std::vector<std::pair<std::vector<cudaEvent_t>, double>> marks;
       size_t marks_seen = 0;
       auto mark = [&] { marks.push_back({h->ev_pending.back().ends, total_steps ? double(done_steps) / double(total_steps) : 1.0}); };
       auto look = [&](bool wait) {
-        for (; marks_seen < marks.size(); ++marks_seen) {
+        for (; marks_seen + (wait ? 1 : 0) < marks.size(); ++marks_seen) {
           for (cudaEvent_t end : marks[marks_seen].first) {
             const cudaError_t e = wait ? cudaEventSynchronize(end) : cudaEventQuery(end);
             if (e == cudaErrorNotReady) cudaGetLastError();
