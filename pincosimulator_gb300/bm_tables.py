@@ -1,7 +1,9 @@
 """Tables of the FP64 Box-Muller draw (csrc/twmc_common.cuh), emitted as
 csrc/bm_tables.inc: table-driven logarithm and sine / cosine in the manner of
-Tang (ACM Trans. Math. Softw. 16, 1990 and 17, 1991), every entry rounded once
-from 60 digits.
+Tang (ACM Trans. Math. Softw. 16, 1990 and 17, 1991), the logarithm's reduction
+that of log in Arm Optimized Routines (math/log.c, MIT licence: offset 0.6875, 128
+intervals of the bit pattern, one of them ending at 1), every entry computed
+here and rounded once from 60 digits.
 
 The uniforms are u = (w + 1/2) 2^-32, w a 32-bit word.
 

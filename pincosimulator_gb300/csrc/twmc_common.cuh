@@ -139,8 +139,8 @@ __host__ __device__ __forceinline__ u32x4 wiener_words(uint32_t pair, uint32_t s
 }
 
 // The Wiener words of one site pair over many steps. Of the ten rounds' twenty
-// 32 x 32 -> 64-bit products (four cycles each on the FMA pipe's wide half,
-// two thirds of the packed steps' time there) the first three rounds hold four
+// 32 x 32 -> 64-bit products (10 of the packed steps' 21.7 instructions on the
+// FMA pipe's wide half, per site) the first three rounds hold four
 // that do not depend on the step and one that all pairs of a trajectory share:
 // a thread keeps what they give per pair (WienerSite) and forms the shared one
 // once per step (WienerStep). The compiler moves these products out of the step
@@ -222,14 +222,19 @@ __device__ __forceinline__ float narrow(double x) {
 __device__ __forceinline__ bool is_zero(double x) { return ((__double2hiint(x) & 0x7fffffff) | __double2loint(x)) == 0; }
 
 // Box-Muller, FP64: u = (w + 1/2) 2^-32, r = sqrt(-2 ln u1), th = 2 pi u2 - pi.
+// The logarithm's reduction (the bit pattern less that of 0.6875, seven bits of
+// it for the interval, an arithmetic shift for the exponent, one interval that
+// ends at 1) is the one of log in Arm Optimized Routines (math/log.c, MIT);
+// tables, polynomial and the rest are this file's and bm_tables.py's.
 // The FP64 pipe of GB300 (two lanes per SM and cycle) bounds FP64 runs, and
 // the general log, sincos and sqrt of a draw were about 70 of its 185
 // instructions per site-update. Here 33: the words' structure makes both
 // argument reductions exact integer work, tables (bm_tables.py) replace most
 // of the polynomials, and the square root refines the FP32 reciprocal root:
 // 500 trajectories of 16x16 over 100 steps take 3.07 ms, before 4.30 ms
-// in all. Errors of the draws against 60 digits over 8192 pairs: rms 0.95e-16,
-// at most 7.5e-16 (with log, sincos and sqrt 1.41e-16 and 1.09e-15).
+// in all. Errors of the draws against 60 digits over 8192 pairs
+// (tests/test_gpu_normals64.py): rms 0.95e-16, at most 7.7e-16 (with log, sincos
+// and sqrt 1.41e-16 and 1.09e-15).
 __device__ __forceinline__ double neg2_log_uniform(uint32_t w) {
   // 2 w + 1 as a double, by its leading bit
   const int lz = w ? __clz(int(w)) : 32;  // 33 - lz significant bits

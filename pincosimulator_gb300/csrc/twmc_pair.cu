@@ -11,10 +11,9 @@ namespace {
 constexpr int64_t kSmemPerSm = 227 * 1024;
 
 // Cycles per warp and slot of a split on a full SM, measured on GB300 with
-// per-site omega (32x32, 64x64, 50x50, 80x80, 1x4096, 128x128 and others): what
-// the FMA pipe's wide half leaves (112 for the packed operations and the
-// Philox products of a pair), the loads a shorter run needs, and the spills of
-// a tighter register cap.
+// per-site omega (32x32, 64x64, 50x50, 80x80, 1x4096, 128x128 and others): a
+// pair's instructions, the loads that a shorter run needs beside them, and
+// the spills of a tighter register cap.
 double slot_cycles(const PairPlan& p) {
   const int s = p.v * p.nb;
   if (p.chain) return s >= 8 ? 125.0 : p.nb > 1 ? 116.0 : 104.0;

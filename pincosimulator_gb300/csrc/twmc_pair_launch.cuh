@@ -21,11 +21,20 @@ struct PairPlan {
 };
 
 // Which 128-register splits keep the step-independent Philox rounds in registers
-// of their own (WienerSite) instead of as the compiler hoists them. GB300, 1e11 site-updates/s without / with: runs of five rows 3.93 / 4.36 (50x50, per-site
-// omega) and 4.00 / 4.30 (scalars); 2 x 2 slots 5.03 / 5.17 (64x64, per-site omega),
-// but 5.32 / 5.23 with scalars; clusters of four 4.15 / 4.25 (128x128, scalars),
-// but 4.24 / 4.16 with per-site omega (120 bytes of spills). One or two slots,
-// chains: the compiler does better by itself (1x64 2.58 / 2.42).
+// of their own (WienerSite) instead of as the compiler hoists them. It pays where
+// the compiler's own hoisting reaches the cap and keeping does not (registers,
+// bytes of spills without / with; GB300, 1e11 site-updates/s without / with):
+//   runs of five rows, per-site omega   128, 4 / 128, 0    3.93 / 4.36 (50x50)
+//                      scalars          128, 12 / 126, 0   4.00 / 4.30
+//   2 x 2 slots, per-site omega         128, 0 / 122, 0    5.03 / 5.17 (64x64)
+//                scalars                124, 0 / 120, 0    5.32 / 5.23
+//   clusters of four, scalars           128, 132 / 128, 60 4.15 / 4.25 (128x128)
+//                     per-site omega    128, 192 / 128, 120 4.24 / 4.16
+//   one slot, chain                     52, 0 / 48, 0      2.58 / 2.42 (1x64)
+// (clusters spill either way, and only measuring told). Not timed by themselves: the
+// other splits of four and more slots, which follow their neighbours here.
+// For a new split: compile both with -Xptxas -v, keep if only that leaves the
+// cap, and time it.
 constexpr bool pair_keep(int v, int nb, bool ch, int par, int cl) {
   if (cl > 1) return par == PAIR_SCALAR;
   return !ch && ((par == PAIR_RSL_IM && v * nb >= 4) || (par == PAIR_SCALAR && v >= 4));

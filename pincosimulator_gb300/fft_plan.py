@@ -252,12 +252,29 @@ def fp64_bits(n: int) -> int:
 
 
 def fp32_bits(n: int) -> int:
-    """Register bits of the FP32 plan of 2^n sites: 16 sites per thread (fewest
-    exchanges), but 8 up to 128 sites, where that costs nothing on a full device
-    and halves a step's latency on a part-filled one. GB300, us per step with 16
-    and 8 sites per thread: 1x32 with 100 trajectories 1.16 / 0.53, with 20000
-    3.30 / 2.07; 1x64 with 1000 1.23 / 0.63, with 16000 4.04 / 4.13; 1x128 with 300
-    1.23 / 0.66, with 8000 3.99 / 3.71; but 1x256 with 6000 5.98 / 11.2."""
+    """Register bits of the FP32 plan of 2^n sites: 16 sites per thread, but 8 up
+    to 128 sites, where that halves a step's latency on a part-filled device.
+    From 256 sites on 8 per thread take twice the passes (1x256, 16x16: 4 for
+    2, 64x64: 6 for 3; up to 128 sites 2 or 3 for 2), and every pass boundary is
+    an exchange each way. GB300, us per step with 4 / 8 / 16 sites per thread
+    (registers 94-128 / 124-198 / 226-255, no spills but on 4 of 1x4096):
+
+        lattice   100 trajectories    1e6 sites in all     4e6 sites            16e6 sites
+        1x32      0.34 0.52 1.14      3.85 2.90 4.14       14.5 10.9 14.6       57.4 43.3 54.7
+        1x64      0.41 0.60 1.22      5.24 4.08 3.99       20.0 15.5 13.8       79.2 61.6 51.7
+        1x128     0.48 0.64 1.21      6.10 3.67 3.96       23.3 13.8 13.7       92.3 54.9 50.9
+        1x256     0.61 0.88 1.21      9.33 7.19 3.98       35.6 27.7 13.8       141 110 51.4
+        1x512     1.07 0.92 1.49      11.7 6.71 5.27       43.7 25.7 18.7       173 98.7 69.5
+        1x1024    1.35 1.31 1.95      7.90 8.06 5.85       29.7 29.3 20.7       119 116 77.2
+        1x4096    7.52 6.32 3.48      15.0 12.6 6.93       52.3 44.0 24.2       194 163 89.7
+        16x16     0.50 0.77 1.06      6.31 5.56 3.56       24.1 21.0 12.4       95.7 83.6 46.0
+        32x32     1.32 0.94 1.34      7.65 4.78 4.68       29.0 18.4 16.3       116 70.5 60.8
+        64x64     5.85 5.25 2.76      11.7 10.5 5.50       40.8 36.5 19.2       151 136 71.2
+
+    The line costs devices that are filled several times over: 1x64 with 16384
+    trajectories 4.19 for 4.00 us, with 250000 61.6 for 51.7. The plan may not
+    depend on the batch: plans do not round alike, so a trajectory's bits
+    would."""
     return 3 if n <= 7 else 4
 
 
