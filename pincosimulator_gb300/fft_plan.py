@@ -60,27 +60,28 @@ class Plan:
         return 1 << (self.nbits - self.e)
 
 
-def _stages_for_dim(dim: int, m: int) -> list:
+def _stages_for_dim(dim: int, m: int, mixed: bool = False) -> list:
     out = []
     t = m
-    while t >= 2:
-        out.append(Stage(dim, t - 2, 2))
-        t -= 2
-    if t == 1:
-        out.append(Stage(dim, 0, 1))
+    while t > 0:
+        rb = 1 if t == 1 or (mixed and out and out[-1].rb == 2) else 2
+        t -= rb
+        out.append(Stage(dim, t, rb))
     return out
 
 
-def make_plan(bx: int, by: int, e: int) -> Plan:
-    """Plan for an (2^bx x 2^by) lattice with 2^e elements per thread."""
+def make_plan(bx: int, by: int, e: int, mixed: bool = False) -> Plan:
+    """Plan for an (2^bx x 2^by) lattice with 2^e elements per thread; `mixed`: radix-4
+    and radix-2 stages in turn (with 8 elements one of each fills a pass, where two
+    radix-4 stages take two)."""
     n = bx + by
     e = min(e, n)
     lo = (0, by)
     m = (by, bx)
     stages = []
     if bx > 0:
-        stages += _stages_for_dim(1, bx)
-    stages += _stages_for_dim(0, by)
+        stages += _stages_for_dim(1, bx, mixed)
+    stages += _stages_for_dim(0, by, mixed)
     # Greedy packing of stages into passes of at most e active bits.
     groups = []
     cur, used = [], 0
@@ -255,13 +256,13 @@ def fp32_bits(n: int) -> int:
     """Register bits of the FP32 plan of 2^n sites: 16 sites per thread, but 8 up
     to 128 sites, where that halves a step's latency on a part-filled device.
     From 256 sites on 8 per thread take twice the passes (1x256, 16x16: 4 for
-    2, 64x64: 6 for 3; up to 128 sites 2 or 3 for 2), and every pass boundary is
+    2, 64x64: 6 for 3; 1x128 3 for 2, below as many), and every pass boundary is
     an exchange each way. GB300, us per step with 4 / 8 / 16 sites per thread
     (registers 94-128 / 124-198 / 226-255, no spills but on 4 of 1x4096):
 
         lattice   100 trajectories    1e6 sites in all     4e6 sites            16e6 sites
         1x32      0.34 0.52 1.14      3.85 2.90 4.14       14.5 10.9 14.6       57.4 43.3 54.7
-        1x64      0.41 0.60 1.22      5.24 4.08 3.99       20.0 15.5 13.8       79.2 61.6 51.7
+        1x64      0.41 0.56 1.22      5.24 3.11 3.99       20.0 11.7 13.8       79.2 46.7 51.7
         1x128     0.48 0.64 1.21      6.10 3.67 3.96       23.3 13.8 13.7       92.3 54.9 50.9
         1x256     0.61 0.88 1.21      9.33 7.19 3.98       35.6 27.7 13.8       141 110 51.4
         1x512     1.07 0.92 1.49      11.7 6.71 5.27       43.7 25.7 18.7       173 98.7 69.5
@@ -271,11 +272,17 @@ def fp32_bits(n: int) -> int:
         32x32     1.32 0.94 1.34      7.65 4.78 4.68       29.0 18.4 16.3       116 70.5 60.8
         64x64     5.85 5.25 2.76      11.7 10.5 5.50       40.8 36.5 19.2       151 136 71.2
 
-    The line costs devices that are filled several times over: 1x64 with 16384
-    trajectories 4.19 for 4.00 us, with 250000 61.6 for 51.7. The plan may not
-    depend on the batch: plans do not round alike, so a trajectory's bits
-    would."""
+    (1x64 with 8: a radix-4 and a radix-2 stage per pass, two passes; three of a
+    radix-4 stage each took 0.60, 4.08, 15.5 and 61.6.) The line costs 1x128 on a
+    device filled several times over: 7.33 for 7.11 us with 16384 trajectories.
+    The plan may not depend on the batch: plans do not round alike, so a
+    trajectory's bits would."""
     return 3 if n <= 7 else 4
+
+
+def fp32_plan(bx: int, by: int) -> Plan:
+    """The FP32 plan of a shape: 64 sites on 8 per thread in two passes (see make_plan)."""
+    return make_plan(bx, by, fp32_bits(bx + by), mixed=(bx, by) == (0, 6))
 
 
 def emit_header() -> str:
@@ -283,7 +290,7 @@ def emit_header() -> str:
     Plan_<bx>_<by> (FP32) and PlanD_<bx>_<by> (FP64)."""
     lines = ["// Generated by pincosimulator_gb300/fft_plan.py -- do not edit.", "#pragma once", "namespace twmc {"]
     for (bx, by) in SUPPORTED_SHAPES:
-        lines += _emit_plan(f"Plan_{bx}_{by}", make_plan(bx, by, fp32_bits(bx + by)))
+        lines += _emit_plan(f"Plan_{bx}_{by}", fp32_plan(bx, by))
     for (bx, by) in SUPPORTED_SHAPES:
         lines += _emit_plan(f"PlanD_{bx}_{by}", make_plan(bx, by, fp64_bits(bx + by)))
     lines.append("}  // namespace twmc")

@@ -50,3 +50,22 @@ def test_short_plans(shape, e):
     ref = np.fft.fft2(x.reshape(1 << shape[0], 1 << shape[1]))
     assert np.abs(fp.run_forward(p, x) - ref[kx, ky]).max() < 1e-10 * np.abs(ref).max()
     assert p.nbits - 1 in p.passes[0].reg and all(len(ps.reg) == e for ps in p.passes)
+
+
+@pytest.mark.parametrize("shape", fp.SUPPORTED_SHAPES)
+def test_fp32_plans(shape):
+    """The FP32 plans as emitted: the transform and its inverse, the layout rules,
+    and no more passes than the bits need."""
+    p = fp.fp32_plan(*shape)
+    rng = np.random.default_rng(4)
+    n = 1 << p.nbits
+    x = rng.normal(size=n) + 1j * rng.normal(size=n)
+    kx, ky = fp.freq_of_position(p)
+    ref = np.fft.fft2(x.reshape(1 << shape[0], 1 << shape[1]))
+    y = fp.run_forward(p, x)
+    assert np.abs(y - ref[kx, ky]).max() < 1e-10 * np.abs(ref).max()
+    assert np.abs(fp.run_inverse(p, y) / n - x).max() < 1e-12
+    assert p.nbits - 1 in p.passes[0].reg
+    for ps in p.passes:
+        assert sorted(ps.reg + ps.thr) == list(range(p.nbits)) and len(ps.reg) == p.e
+    assert len(p.passes) == -(-p.nbits // p.e)
