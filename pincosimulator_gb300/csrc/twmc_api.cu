@@ -197,6 +197,7 @@ bool upload_raw(twmc_handle* h, DevBuf* b, std::vector<T> v) {
   return cudaMemcpyAsync(b->p, kept->data(), bytes, cudaMemcpyHostToDevice, h->stream) == cudaSuccess;
 }
 
+constexpr size_t kMostUploads = 64;  // kept before a new batch waits for the earlier ones
 // Waits for the handle's stream; the sources of its uploads are free then.
 cudaError_t settle(twmc_handle* h) {
   const cudaError_t e = cudaStreamSynchronize(h->stream);
@@ -434,7 +435,6 @@ int build_tables(twmc_handle* h) {
     }
     if (!upload_c(h, &h->d_shared_par[k], std::move(v))) return fail(h, TWMC_ERR_NOMEM, "parameter upload");
   }
-  TWMC_CUDA(h, settle(h));
   return TWMC_OK;
 }
 
@@ -581,7 +581,7 @@ int reduce(twmc_handle* h) {
 int batch_init(twmc_handle* h, const twmc_task_desc* tasks, size_t n, const bool (&want_real)[3]) {
   const int64_t N = h->nsites;
   const int prec = h->prec;
-  if (!h->uploads.empty()) TWMC_CUDA(h, settle(h));  // (a batch that nothing has waited for)
+  if (h->uploads.size() >= kMostUploads) TWMC_CUDA(h, settle(h));  // (batches that nothing has waited for)
   h->ntraj = int64_t(n);
   h->step_pos = 0;
   const size_t c2 = 2 * rsize(prec);

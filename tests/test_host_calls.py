@@ -74,6 +74,9 @@ for prec in (twmc.PREC_F32, twmc.PREC_F64):
         s.run(t, realizations=True)
         s.run(t, moments=True)
         s.batch_init(t); s.advance(3); s.batch_init(t); s.advance(3); s.reduce(); s.sync()
+        for _ in range(40):
+            s.batch_init(t); s.advance(1)
+        s.sync()
         s.close()
     s, t = square(precision=prec, noise=twmc.NOISE_BUFFER)
     s.set_noise(c(5, 4, 256))
@@ -84,7 +87,7 @@ for prec in (twmc.PREC_F32, twmc.PREC_F64):
                     U=c(24), F_t=(times, c(len(times), 24)))
     s.run(s.make_tasks(3, t_end=0.04))
     s.close()
-assert lib.fake_uploads() > 60, lib.fake_uploads()
+assert lib.fake_uploads() > 600, lib.fake_uploads()
 assert lib.fake_changed() == 0, (lib.fake_changed(), lib.fake_uploads())
 """)
 
