@@ -126,6 +126,7 @@ struct twmc_handle {
   size_t h_stage_bytes = 0;
   // host sources of the uploads since the stream was last waited for
   std::vector<std::shared_ptr<void>> uploads;
+  size_t upload_bytes = 0;
   std::vector<double> ft_times;   // with sentinel
   std::vector<cd> ft_vals, ft_slopes;
   // kernel selection
@@ -187,22 +188,24 @@ size_t rsize(int prec) { return prec ? sizeof(double) : sizeof(float); }
 // Uploads go on the handle's stream, in order with the kernels that read them.
 // A copy from pageable memory may return before it has read its source (on a
 // host whose memory the GPU reads coherently nothing need be staged), so the
-// handle keeps the source until the stream has been waited for.
+// handle keeps the source until the stream has been waited for; it waits itself
+// before it keeps much.
+constexpr size_t kMostUploads = 64, kMostUploadBytes = size_t(1) << 26;
+// Waits for the handle's stream; the sources of its uploads are free then.
+cudaError_t settle(twmc_handle* h) {
+  const cudaError_t e = cudaStreamSynchronize(h->stream);
+  if (e == cudaSuccess) { h->uploads.clear(); h->upload_bytes = 0; }
+  return e;
+}
 template <typename T>
 bool upload_raw(twmc_handle* h, DevBuf* b, std::vector<T> v) {
   const size_t bytes = v.size() * sizeof(T);
   if (!b->ensure(bytes)) return false;
   auto kept = std::make_shared<std::vector<T>>(std::move(v));
   h->uploads.push_back(kept);
-  return cudaMemcpyAsync(b->p, kept->data(), bytes, cudaMemcpyHostToDevice, h->stream) == cudaSuccess;
-}
-
-constexpr size_t kMostUploads = 64;  // kept before a new batch waits for the earlier ones
-// Waits for the handle's stream; the sources of its uploads are free then.
-cudaError_t settle(twmc_handle* h) {
-  const cudaError_t e = cudaStreamSynchronize(h->stream);
-  if (e == cudaSuccess) h->uploads.clear();
-  return e;
+  h->upload_bytes += bytes;
+  if (cudaMemcpyAsync(b->p, kept->data(), bytes, cudaMemcpyHostToDevice, h->stream) != cudaSuccess) return false;
+  return (h->uploads.size() < kMostUploads && h->upload_bytes < kMostUploadBytes) || settle(h) == cudaSuccess;
 }
 
 // Upload complex values in the state precision.
@@ -581,7 +584,6 @@ int reduce(twmc_handle* h) {
 int batch_init(twmc_handle* h, const twmc_task_desc* tasks, size_t n, const bool (&want_real)[3]) {
   const int64_t N = h->nsites;
   const int prec = h->prec;
-  if (h->uploads.size() >= kMostUploads) TWMC_CUDA(h, settle(h));  // (batches that nothing has waited for)
   h->ntraj = int64_t(n);
   h->step_pos = 0;
   const size_t c2 = 2 * rsize(prec);

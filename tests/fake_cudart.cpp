@@ -38,7 +38,7 @@ std::map<const void*, std::string>& names() { static std::map<const void*, std::
 std::map<const void*, int>& smem() { static std::map<const void*, int> m; return m; }
 std::map<char*, size_t>& pinned() { static std::map<char*, size_t> m; return m; }
 size_t pinned_now = 0, pinned_peak = 0, pinned_limit = ~size_t(0);
-long g_uploads = 0, g_changed = 0, g_lowered = 0, g_launches = 0, g_fail_at = -1;
+long g_uploads = 0, g_queued = 0, g_queued_most = 0, g_changed = 0, g_lowered = 0, g_launches = 0, g_fail_at = -1;
 std::string g_fail_name, g_log;
 std::map<std::string, double>& costs() { static std::map<std::string, double> m; return m; }
 double cost(const std::string& name) {
@@ -80,6 +80,7 @@ extern "C" {
 // ---- controls ----
 long fake_uploads() { return g_uploads; }           // copies from pageable memory that have run
 long fake_changed() { return g_changed; }           // of those, with another source than when they were issued
+long fake_queued_most() { return g_queued_most; }   // largest sum of their bytes that had not run
 long fake_lowered() { return g_lowered; }           // dynamic shared-memory limits set below an earlier value
 size_t fake_pinned_peak() { return pinned_peak; }
 void fake_pinned_limit(size_t n) { pinned_limit = n; pinned_peak = pinned_now; }
@@ -191,8 +192,11 @@ cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind k, 
   if (n && k != cudaMemcpyDeviceToDevice && is_pinned(host) != is_pinned(host + n - 1)) return ret(cudaErrorInvalidValue);
   if (k == cudaMemcpyHostToDevice && !is_pinned(s)) {
     std::string was(static_cast<const char*>(s), n);
+    g_queued += long(n);
+    if (g_queued > g_queued_most) g_queued_most = g_queued;
     push(of(st), [=] {
       ++g_uploads;
+      g_queued -= long(n);
       if (std::memcmp(s, was.data(), n) != 0) ++g_changed;
       std::memcpy(d, s, n);
     });

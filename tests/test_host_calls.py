@@ -15,7 +15,7 @@ import ctypes as C
 import numpy as np
 from pincosimulator_gb300 import twmc
 lib = twmc.load()
-for f in ("fake_uploads", "fake_changed", "fake_lowered"):
+for f in ("fake_uploads", "fake_changed", "fake_lowered", "fake_queued_most"):
     getattr(lib, f).restype = C.c_long
 lib.fake_pinned_peak.restype = C.c_size_t
 lib.fake_pinned_limit.argtypes = [C.c_size_t]
@@ -306,4 +306,20 @@ for n_traj in (4000, 1, 300):
 for shapes in ([(64, 64), (128, 128)], [(6, 10), (80, 80), (25, 25)], [(128, 128), (96, 96)], [(50, 50)], [(120, 100)]):
     twmc.HBatch([dict(nx=nx, ny=ny, dt=0.01, n_traj=3) for nx, ny in shapes], 10).close()
 assert lib.fake_lowered() == 0, lib.fake_lowered()
+""")
+
+
+def test_kept_sources_are_bounded(script):
+    """Batches that nothing waits for: their uploads' sources do not pile up."""
+    script("""
+rng = np.random.default_rng(2)
+s = twmc.System(nx=64, ny=64, J=1.0, dt=0.01, frame_steps=2)
+f = rng.normal(size=(100, 4096)) + 1j * rng.normal(size=(100, 4096))   # 6.6 MB
+t = s.make_tasks(100, ic=twmc.IC_GIVEN, init_field=f)
+for _ in range(40):
+    s.batch_init(t)
+    s.advance(1)
+assert lib.fake_changed() == 0
+assert lib.fake_queued_most() < (1 << 26) + (1 << 23), lib.fake_queued_most()
+s.close()
 """)
