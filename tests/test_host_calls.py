@@ -1,7 +1,6 @@
 """Host code of the library on the CPU, linked with a stand-in for the CUDA
 runtime (fake_cudart.cpp) whose streams run their work as late as the runtime
 allows. Each test runs a script in a process of its own."""
-import glob
 import os
 import subprocess
 import sys
@@ -39,6 +38,8 @@ def fake_lib(built_lib, tmp_path_factory):
     from pincosimulator_gb300 import build_ext
 
     objs = [os.path.join(build_ext.BUILD, s.replace(".cu", ".o")) for s in build_ext.SOURCES]
+    if not all(map(os.path.exists, objs)):
+        build_ext.build(force=True)
     subprocess.run(["g++", "-shared", "-Wl,-Bsymbolic", "-Wl,--no-undefined", *objs, obj, "-o", lib], check=True)
     return lib
 
